@@ -2,7 +2,6 @@
 // the interface of SKIRT's PathSegmentGenerator (start / next / m / ds). The *Exact walkers keep
 // the reference generators' FP64 operation order with separate roundings, so that for identical
 // rays they return the same cell sequences and segment lengths as the CPU code:
-//   CartesianExact  <- CartesianSpatialGrid::MySegmentGenerator::next   (CartesianSpatialGrid.cpp:77-155)
 //   OctreeExact     <- TreeSpatialGrid::MySegmentGenerator::next        (TreeSpatialGrid.cpp:143-228)
 //   AdaptiveMeshExact <- AdaptiveMeshSnapshot::MySegmentGenerator::next (AdaptiveMeshSnapshot.cpp:378-449)
 //   VoronoiExact    <- VoronoiMeshSnapshot::MySegmentGenerator::next    (VoronoiMeshSnapshot.cpp:1089-1222)
@@ -29,6 +28,9 @@ struct GridDev
     const double* yb;
     const double* zb;
     int nx, ny, nz;
+    // the walls a ray meets one after the other, per axis upwards (the borders) and downwards (the
+    // negated borders in reverse), each sequence followed by a NaN
+    const double* cWall;
 
     // octree: per node bounds (6 doubles), cell index (-1 non-leaf), first child (-1 leaf),
     // neighbour CSR per (node, wall)
@@ -47,7 +49,8 @@ struct GridDev
     // leaf-indexed 64-byte records of the production walker (four int4 per cell):
     //   [0] wall indices x lo|hi<<16, y, z (16 bits each, into the lattice wall tables), FP32 density
     //   [1] neighbour-list base, 9-bit cumulative wall offsets (64 bits), leaf node id
-    //   [2] [3] per wall the single positive-overlap neighbour (-1: domain wall, -2: scan the list)
+    //   [2] [3] per wall the single positive-overlap neighbour (-1: domain wall, -2: scan the list),
+    //       FP64 density
     // and the positive-overlap neighbour lists (overlap-sorted, cell indices) of every leaf wall
     const int4* tRec;
     const int* tLeafNb;
@@ -237,70 +240,6 @@ SKG_D double boxDiagonal(const double* b)
     double dx = xsub(b[3], b[0]), dy = xsub(b[4], b[1]), dz = xsub(b[5], b[2]);
     return sqrt(xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz)));
 }
-
-// ---------------------------------------------------------------------------------------------
-// Cartesian
-// ---------------------------------------------------------------------------------------------
-struct CartesianExact : GenBase
-{
-    static constexpr int kMinBlocks = 3;
-    static constexpr int kRefillMin = 16;  // waiting lanes before a warp takes new tasks
-    int i, j, k;
-
-    SKG_D void start(const GridDev&, double x, double y, double z, double ux, double uy, double uz, int = -1)
-    {
-        startRay(x, y, z, ux, uy, uz);
-    }
-
-    SKG_D bool next(const GridDev& g)
-    {
-        if (state == GS_OUTSIDE) return false;
-        if (state == GS_UNKNOWN)
-        {
-            if (!moveInside(g.ext, xmul(1e-12, boxDiagonal(g.ext)))) return false;
-            i = locateClip(g.xb, g.nx + 1, rx);
-            j = locateClip(g.yb, g.ny + 1, ry);
-            k = locateClip(g.zb, g.nz + 1, rz);
-            if (ds > 0.) return true;
-        }
-        // state == inside
-        int mm = k + g.nz * j + g.nz * g.ny * i;
-        double xE = (kx < 0.0) ? g.xb[i] : g.xb[i + 1];
-        double yE = (ky < 0.0) ? g.yb[j] : g.yb[j + 1];
-        double zE = (kz < 0.0) ? g.zb[k] : g.zb[k + 1];
-        double dsx = (fabs(kx) > 1e-15) ? xsub(xE, rx) / kx : DBL_MAX;
-        double dsy = (fabs(ky) > 1e-15) ? xsub(yE, ry) / ky : DBL_MAX;
-        double dsz = (fabs(kz) > 1e-15) ? xsub(zE, rz) / kz : DBL_MAX;
-        if (dsx <= dsy && dsx <= dsz)
-        {
-            m = mm; ds = dsx;
-            rx = xE;
-            ry = xadd(ry, xmul(ky, dsx));
-            rz = xadd(rz, xmul(kz, dsx));
-            i += (kx < 0.0) ? -1 : 1;
-            if (i >= g.nx || i < 0) state = GS_OUTSIDE;
-        }
-        else if (dsy < dsx && dsy <= dsz)
-        {
-            m = mm; ds = dsy;
-            ry = yE;
-            rx = xadd(rx, xmul(kx, dsy));
-            rz = xadd(rz, xmul(kz, dsy));
-            j += (ky < 0.0) ? -1 : 1;
-            if (j >= g.ny || j < 0) state = GS_OUTSIDE;
-        }
-        else
-        {
-            m = mm; ds = dsz;
-            rz = zE;
-            rx = xadd(rx, xmul(kx, dsz));
-            ry = xadd(ry, xmul(ky, dsz));
-            k += (kz < 0.0) ? -1 : 1;
-            if (k >= g.nz || k < 0) state = GS_OUTSIDE;
-        }
-        return true;
-    }
-};
 
 // ---------------------------------------------------------------------------------------------
 // Octree

@@ -4,6 +4,7 @@
 // sums, GpuAcceleration.hpp), and they are what the cell-sequence parity tests call.
 #include "internal.hpp"
 #include "paths.cuh"
+#include "grids_fast.cuh"
 
 namespace skg {
 
@@ -15,8 +16,13 @@ cudaError_t launchTracePathsFP64(int precision, const GridDev& g, int n, const d
     (void)precision;
     switch (g.kind)
     {
-        case 0: tracePathsKernel<CartesianExact><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err); break;
-        case 1: tracePathsKernel<OctreeExact><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err); break;
+        case 0: tracePathsKernel<CartesianT<double>><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err); break;
+        case 1:
+            if (g.tWallN)
+                tracePathsKernel<OctreeT<double>><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err);
+            else
+                tracePathsKernel<OctreeExact><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err);
+            break;
         case 2: tracePathsKernel<VoronoiExact><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err); break;
         case 3: tracePathsKernel<TetraExact><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err); break;
         case 4: tracePathsKernel<Sphere1DExact><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err); break;
@@ -38,8 +44,13 @@ cudaError_t launchOpticalDepthsFP64(int precision, const GridDev& g, const doubl
     (void)precision;
     switch (g.kind)
     {
-        case 0: opticalDepthKernel<CartesianExact><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err); break;
-        case 1: opticalDepthKernel<OctreeExact><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err); break;
+        case 0: opticalDepthKernel<CartesianT<double>><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err); break;
+        case 1:
+            if (g.tWallN)
+                opticalDepthKernel<OctreeT<double>><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err);
+            else
+                opticalDepthKernel<OctreeExact><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err);
+            break;
         case 2: opticalDepthKernel<VoronoiExact><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err); break;
         case 3: opticalDepthKernel<TetraExact><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err); break;
         case 4: opticalDepthKernel<Sphere1DExact><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err); break;

@@ -15,10 +15,10 @@ cudaError_t launchTracePathsFP32(int precision, const GridDev& g, int n, const d
     (void)precision;
     switch (g.kind)
     {
-        case 0: tracePathsKernel<CartesianFast><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err); break;
+        case 0: tracePathsKernel<CartesianT<float>><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err); break;
         case 1:
             if (g.tWallN)
-                tracePathsKernel<OctreeRec><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err);
+                tracePathsKernel<OctreeT<float>><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err);
             else
                 tracePathsKernel<OctreeNodeFast><<<blocks, threads, 0, s>>>(g, n, rays, maxSeg, count, m, ds, err);
             break;
@@ -43,10 +43,10 @@ cudaError_t launchOpticalDepthsFP32(int precision, const GridDev& g, const doubl
     (void)precision;
     switch (g.kind)
     {
-        case 0: opticalDepthKernel<CartesianFast><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err); break;
+        case 0: opticalDepthKernel<CartesianT<float>><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err); break;
         case 1:
             if (g.tWallN)
-                opticalDepthKernel<OctreeRec><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err);
+                opticalDepthKernel<OctreeT<float>><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err);
             else
                 opticalDepthKernel<OctreeNodeFast><<<blocks, threads, 0, s>>>(g, dens, section, n, rays, tau, err);
             break;

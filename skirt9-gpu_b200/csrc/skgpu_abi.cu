@@ -129,11 +129,15 @@ bool finiteAll(const double* v, size_t n)
     return true;
 }
 
-// copies the number densities into the FP32 leaf records of an octree grid (4 float4 per leaf)
+// copies the number densities into the leaf records of an octree grid (four int4 per leaf): FP32 in
+// the last word of the first int4, FP64 in the second half of the last
 __global__ void fillLeafDensityKernel(int4* rec, const double* dens, int n)
 {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < n) rec[4 * static_cast<size_t>(c)].w = __float_as_int(static_cast<float>(dens[c]));
+    if (c >= n) return;
+    int4* r = rec + 4 * static_cast<size_t>(c);
+    r[0].w = __float_as_int(static_cast<float>(dens[c]));
+    reinterpret_cast<double*>(r + 3)[1] = dens[c];
 }
 
 int syncLeafDensity(skgpu_ctx* ctx)
@@ -367,10 +371,26 @@ int skgpu_upload_grid_cartesian(skgpu_ctx* ctx, const double* xb, int32_t nxb, c
     long long nc = 1LL * g.nx * g.ny * g.nz;
     if (nc > 2147483647LL) return fail(ctx, SKGPU_ERR_ARG, "too many cells");
     g.numCells = static_cast<int>(nc);
+    // the step by which CartesianSpatialGrid moves a ray inside: 1e-12 of the domain's diagonal
+    const double dx = g.ext[3] - g.ext[0], dy = g.ext[4] - g.ext[1], dz = g.ext[5] - g.ext[2];
+    g.eps = 1e-12 * std::sqrt(dx * dx + dy * dy + dz * dz);
+    // the walls in the order in which a ray meets them, for either direction of each axis
+    std::vector<double> walls;
+    auto addWalls = [&](const double* v, int n) {
+        const double end = std::numeric_limits<double>::quiet_NaN();
+        walls.insert(walls.end(), v, v + n);
+        walls.push_back(end);
+        for (int i = n - 1; i >= 0; --i) walls.push_back(-v[i]);
+        walls.push_back(end);
+    };
+    addWalls(xb, nxb);
+    addWalls(yb, nyb);
+    addWalls(zb, nzb);
     int rc;
     if ((rc = gridUpload(ctx, &g.xb, xb, nxb))) return rc;
     if ((rc = gridUpload(ctx, &g.yb, yb, nyb))) return rc;
     if ((rc = gridUpload(ctx, &g.zb, zb, nzb))) return rc;
+    if ((rc = gridUpload<double>(ctx, &g.cWall, walls.data(), walls.size()))) return rc;
     ctx->hasGrid = true;
     return SKGPU_OK;
 }
@@ -641,7 +661,7 @@ int skgpu_upload_grid_octree(skgpu_ctx* ctx, int32_t num_nodes, const double* bo
     //   [1] neighbour-list base, the 9-bit cumulative offsets of the 6 walls in the list (64 bits, all
     //       ones: no list), the leaf's node id (for the full neighbour lists of the exact fallback)
     //   [2] [3] per wall the one neighbour across it when there is exactly one (-1: no neighbour, the
-    //       domain wall; -2: several, scan the list), two spare words
+    //       domain wall; -2: several, scan the list), FP64 density (filled with the FP32 one)
     // The lists hold per wall the positive-overlap neighbours in the reference's overlap order;
     // zero-overlap entries, which only touch an edge, come last in the reference's lists (TreeNode
     // sortNeighbors, TreeNode.cpp:200-207) and are left to the walker's exact fallback.

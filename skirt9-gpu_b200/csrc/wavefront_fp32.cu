@@ -13,9 +13,9 @@ cudaError_t runWaveFP32(int gridKind, const Wave& w, int numSMs, cudaStream_t s,
 {
     switch (gridKind)
     {
-        case 0: return runWave<CartesianFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
+        case 0: return runWave<CartesianT<float>>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
         case 1:
-            return w.sc.g.tWallN ? runWave<OctreeRec>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache)
+            return w.sc.g.tWallN ? runWave<OctreeT<float>>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache)
                                  : runWave<OctreeNodeFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
         case 2: return runWave<VoronoiRec32>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
         case 3: return runWave<TetraPlane32>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);

@@ -2,6 +2,7 @@
 // Compiled with --fmad=false so that the FP64 physics outside the walkers (weights, directions,
 // positions) is rounded like the reference CPU build (x86-64 SSE2, no FMA).
 #include "internal.hpp"
+#include "grids_fast.cuh"
 #include "wavefront_driver.cuh"
 
 namespace skg {
@@ -12,8 +13,10 @@ cudaError_t runWaveFP64(int gridKind, const Wave& w, int numSMs, cudaStream_t s,
 {
     switch (gridKind)
     {
-        case 0: return runWave<CartesianExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 1: return runWave<OctreeExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
+        case 0: return runWave<CartesianT<double>>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
+        case 1:
+            return w.sc.g.tWallN ? runWave<OctreeT<double>>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache)
+                                 : runWave<OctreeExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
         case 2: return runWave<VoronoiExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
         case 3: return runWave<TetraExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
         case 4: return runWave<Sphere1DExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
