@@ -137,8 +137,9 @@ static_assert(sizeof(TetRec) == 128, "one cache line per tetrahedron");
 struct GenBase
 {
     using Acc = double;  // accumulator type of optical depth and path length along the walk
-    // the wavefront runs peel-off and propagation rays as two concurrent traversal kernels
-    static constexpr bool kSplit = true;
+    // the cell of a launched packet is found once, by the launch stage, instead of by each of its rays
+    static constexpr bool kLocates = false;
+    SKG_D static int locate(const GridDev&, double, double, double) { return -1; }
     double rx, ry, rz, kx, ky, kz;
     double ds;
     int m;

@@ -201,6 +201,7 @@ struct OctreeT : BoxWalker
 
     SKG_D double density(const double*) const { return static_cast<double>(segDens); }
 
+    static constexpr bool kLocates = true;
     SKG_D static int locate(const GridDev& g, double x, double y, double z)
     {
         int n = octreeLeafChild(g, x, y, z);
@@ -407,12 +408,10 @@ SKG_D int voronoiLocate(const GridDev& g, double x, double y, double z)
 // Voronoi mesh, production walker (VoronoiMeshSnapshot::MySegmentGenerator::next,
 // VoronoiMeshSnapshot.cpp:1089-1222). Each cell is one contiguous record in 16-byte units:
 //   [0] site x, y (FP64)   [1] site z (FP64), cell index, face count n
-//   [2, 2 + n4)            per face the outward unit normal n and the distance d of the face's plane
-//                          from the site (half the site distance, or the distance to a domain wall)
-//   [2 + n4, 2 + n4 + n4/4) per face the neighbour's record offset (16-byte units), or the wall id
-//                          -1..-6, or kPad
-// with n4 = n rounded up to a multiple of 4 (padding faces have n = 0 and are never ahead). A
-// crossing reads one record and takes the next cell's offset from it: no index arrays between
+//   then per group of four faces five units: for each face the outward unit normal n and the
+//   distance d of the face's plane from the site (half the site distance, or the distance to a domain
+//   wall), and the four neighbours' record offsets (16-byte units), or the wall id -1..-6, or kPad
+// (padding faces have n = 0 and are never ahead). A crossing reads one record and takes the next cell's offset from it: no index arrays between
 // cells. On entering a cell the FP64 position is rebased to FP32 coordinates l relative to the
 // site; the exit through a face is s = (d - n . l) / (n . k). The two smallest exits are
 // re-decided in FP64 from the exact sites when they lie within a near-tie tolerance (FP32 would
@@ -421,21 +420,14 @@ SKG_D int voronoiLocate(const GridDev& g, double x, double y, double z)
 // nearest-site search. A start in a known cell (a scattering event's interaction cell) needs no
 // search; other starts walk greedily over the Delaunay neighbours from a site of the search block.
 // ---------------------------------------------------------------------------------------------
-#ifndef SKG_VORONOI32_MIN_BLOCKS
-#define SKG_VORONOI32_MIN_BLOCKS 3
-#endif
-#ifndef SKG_VORONOI32_REFILL
-#define SKG_VORONOI32_REFILL 8
-#endif
 struct VoronoiRec32 : GenBase
 {
     using Acc = float;
-    static constexpr int kMinBlocks = SKG_VORONOI32_MIN_BLOCKS;
-    static constexpr int kRefillMin = SKG_VORONOI32_REFILL;  // waiting lanes before a warp takes new tasks
-    // one traversal kernel: the Voronoi walk's register footprint leaves no room for two resident
-    // kernels (4.62e6 packets/s unsplit against 4.41e6 split on the Voronoi galaxy)
-    static constexpr bool kSplit = false;
-    static constexpr int kNone = -99;     // no previous cell (the wall ids -1..-6 are taken)
+    // Two blocks per SM and 128 registers for the two groups of faces in flight: the walk waits on
+    // loads, not on warps (galaxy on 1e5 sites, 2e6 packets: 150 ms; three blocks 166 ms, four 199 ms)
+    static constexpr int kMinBlocks = 2;
+    static constexpr int kRefillMin = 8;  // waiting lanes before a warp takes new tasks
+    static constexpr int kNone = -99;     // no previous cell, no exit (the wall ids -1..-6 are taken)
     static constexpr int kPad = -100;     // padding face
     int rec, prev;                        // record offsets of the current and the previous cell
     float kxf, kyf, kzf;
@@ -485,6 +477,9 @@ struct VoronoiRec32 : GenBase
         return 0.;
     }
 
+    static constexpr bool kLocates = true;
+    SKG_D static int locate(const GridDev& g, double x, double y, double z) { return voronoiLocate(g, x, y, z); }
+
     SKG_D bool locateRec(const GridDev& g, int cellHint)
     {
         int c = cellHint >= 0 ? cellHint : voronoiLocate(g, rx, ry, rz);
@@ -508,50 +503,59 @@ struct VoronoiRec32 : GenBase
         }
         for (int guard = 0; guard < 64; ++guard)
         {
+            // the loads of a group of faces are issued together, and those of the next group before the
+            // present one is worked on: the walk waits on record loads that miss L1 more than on anything
+            // else
             const float4* R = g.vRec + rec;
             float4 h0 = __ldg(R), h1 = __ldg(R + 1);
+            const float4* E = R + 2;
+            float4 q[4] = {__ldg(E), __ldg(E + 1), __ldg(E + 2), __ldg(E + 3)};
+            float4 ids = __ldg(E + 4);
             // the FP64 site only rebases the position here (the near-tie branch reloads it)
             float lx = static_cast<float>(rx - __hiloint2double(__float_as_int(h0.y), __float_as_int(h0.x)));
             float ly = static_cast<float>(ry - __hiloint2double(__float_as_int(h0.w), __float_as_int(h0.z)));
             float lz = static_cast<float>(rz - __hiloint2double(__float_as_int(h1.y), __float_as_int(h1.x)));
             int cell = __float_as_int(h1.z);
-            int n4 = (__float_as_int(h1.w) + 3) & ~3;
-            const float4* E = R + 2;
-            const int4* ids = reinterpret_cast<const int4*>(R + 2 + n4);
+            const int n = __float_as_int(h1.w);
             // the two nearest exits me / nk, compared by cross-multiplication so that only those two
-            // distances take a division
-            float meB = 0.f, nkB = 1.f, meS = 0.f, nkS = 1.f, scale = 0.f;
+            // distances take a division, without branches (a face is ahead or not as good as at random, so
+            // that a branch leaves half the lanes idle); none yet is the fraction inf / 1
+            float meB = INFINITY, nkB = 1.f, meS = INFINITY, nkS = 1.f, scale = 0.f;
             int ib = kNone, is = kNone;
-            for (int c = 0; c < n4; c += 4)
+            for (int c = n;;)
             {
-                // four faces per step: their loads are issued together
-                float4 q[4] = {__ldg(E + c), __ldg(E + c + 1), __ldg(E + c + 2), __ldg(E + c + 3)};
-                int4 id4 = __ldg(ids + (c >> 2));
-                int id[4] = {id4.x, id4.y, id4.z, id4.w};
+                float4 qn[4], idn;
+                c -= 4;
+                E += 5;
+                if (c > 0)
+                {
+                    qn[0] = __ldg(E);
+                    qn[1] = __ldg(E + 1);
+                    qn[2] = __ldg(E + 2);
+                    qn[3] = __ldg(E + 3);
+                    idn = __ldg(E + 4);
+                }
+                const int id[4] = {__float_as_int(ids.x), __float_as_int(ids.y), __float_as_int(ids.z), __float_as_int(ids.w)};
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                 {
-                    float nk = q[j].x * kxf + q[j].y * kyf + q[j].z * kzf;
-                    if (!(nk > 0.f) || id[j] == prev) continue;
-                    float me = q[j].w - (q[j].x * lx + q[j].y * ly + q[j].z * lz);
-                    if (!(me > 0.f)) continue;
-                    if (ib == kNone || me * nkB < meB * nk)
-                    {
-                        meS = meB;
-                        nkS = nkB;
-                        is = ib;
-                        meB = me;
-                        nkB = nk;
-                        ib = id[j];
-                        scale = q[j].w;
-                    }
-                    else if (is == kNone || me * nkS < meS * nk)
-                    {
-                        meS = me;
-                        nkS = nk;
-                        is = id[j];
-                    }
+                    const float nk = q[j].x * kxf + q[j].y * kyf + q[j].z * kzf;
+                    const float me = q[j].w - (q[j].x * lx + q[j].y * ly + q[j].z * lz);
+                    const bool ahead = (nk > 0.f) & (me > 0.f) & (id[j] != prev);
+                    const bool b = ahead & (me * nkB < meB * nk);
+                    const bool s = ahead & (me * nkS < meS * nk);
+                    meS = b ? meB : (s ? me : meS);
+                    nkS = b ? nkB : (s ? nk : nkS);
+                    is = b ? ib : (s ? id[j] : is);
+                    meB = b ? me : meB;
+                    nkB = b ? nk : nkB;
+                    ib = b ? id[j] : ib;
+                    scale = b ? q[j].w : scale;
                 }
+                if (c <= 0) break;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) q[j] = qn[j];
+                ids = idn;
             }
             if (ib == kNone)
             {
@@ -699,6 +703,9 @@ struct TetraPlane32 : GenBase
         kyf = static_cast<float>(uy);
         kzf = static_cast<float>(uz);
     }
+
+    static constexpr bool kLocates = true;
+    SKG_D static int locate(const GridDev& g, double x, double y, double z) { return tetraLocate(g, x, y, z); }
 
     // whether the float exit decision in tetrahedron r may differ from the exact one: the point lies
     // within tol of the exit plane, the two nearest exits lie within the planes' error of each other

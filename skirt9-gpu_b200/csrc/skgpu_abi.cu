@@ -818,7 +818,7 @@ int skgpu_upload_grid_voronoi(skgpu_ctx* ctx, int32_t num_sites, const double* s
     // count, then per face the outward unit normal and the distance of the face's plane from the site
     // (half the site distance for a neighbour, the distance to the domain wall for a wall), so that
     // s = (d - n . l) / (n . k) needs no squares of metre-scale coordinates, then per face the
-    // neighbour's record offset (or the wall id); the faces are padded to a multiple of 4
+    // neighbour's record offset (or the wall id); faces and offsets in groups of four faces, padded
     // The records are laid out in the Morton order of their sites (21 bits per axis over the
     // domain), not in cell order: a record spans several cache lines, and cells that are close in
     // space (and so visited together) then share lines and DRAM pages. Only the layout changes;
@@ -856,7 +856,7 @@ int skgpu_upload_grid_voronoi(skgpu_ctx* ctx, int32_t num_sites, const double* s
         int c = layout[q];
         size_t n4 = (static_cast<size_t>(nb_begin[c + 1] - nb_begin[c]) + 3) & ~static_cast<size_t>(3);
         recOff[c] = static_cast<int>(units);
-        units += 2 + n4 + n4 / 4;
+        units += 2 + std::max<size_t>(n4, 4) + std::max<size_t>(n4, 4) / 4;  // a walk reads the first group unasked
         if (units > 2147483647ULL) return fail(ctx, SKGPU_ERR_ARG, "voronoi: mesh too large for 32-bit record offsets");
     }
     std::vector<float4> rec(units);
@@ -865,7 +865,7 @@ int skgpu_upload_grid_voronoi(skgpu_ctx* ctx, int32_t num_sites, const double* s
         const double* pc = sites + 3 * static_cast<size_t>(c);
         float4* R = rec.data() + recOff[c];
         int nf = nb_begin[c + 1] - nb_begin[c];
-        int n4 = (nf + 3) & ~3;
+        int n4 = std::max((nf + 3) & ~3, 4);
         double* hd = reinterpret_cast<double*>(R);
         hd[0] = pc[0];
         hd[1] = pc[1];
@@ -873,15 +873,13 @@ int skgpu_upload_grid_voronoi(skgpu_ctx* ctx, int32_t num_sites, const double* s
         int* hi = reinterpret_cast<int*>(R + 1);
         hi[2] = c;
         hi[3] = nf;
-        int* ids = reinterpret_cast<int*>(R + 2 + n4);
         for (int j = 0; j < n4; ++j)
         {
-            if (j >= nf)
-            {
-                R[2 + j] = make_float4(0.f, 0.f, 0.f, 0.f);
-                ids[j] = -100;  // padding face: never ahead
-                continue;
-            }
+            float4& face = R[2 + j + j / 4];
+            int& id = reinterpret_cast<int*>(R + 2 + 5 * (j / 4) + 4)[j % 4];
+            face = make_float4(0.f, 0.f, 0.f, 0.f);
+            id = -100;  // padding face: never ahead
+            if (j >= nf) continue;
             int mi = nb_index[nb_begin[c] + j];
             double n[3] = {0, 0, 0}, d = 0;
             if (mi >= 0)
@@ -892,7 +890,7 @@ int skgpu_upload_grid_voronoi(skgpu_ctx* ctx, int32_t num_sites, const double* s
                 if (len > 0)
                     for (int a = 0; a < 3; ++a) n[a] /= len;
                 d = 0.5 * len;
-                ids[j] = recOff[mi];
+                id = recOff[mi];
             }
             else
             {
@@ -900,10 +898,10 @@ int skgpu_upload_grid_voronoi(skgpu_ctx* ctx, int32_t num_sites, const double* s
                 bool upper = ((-mi - 1) & 1) != 0;
                 n[a] = upper ? 1.0 : -1.0;
                 d = upper ? extent[3 + a] - pc[a] : pc[a] - extent[a];
-                ids[j] = mi;
+                id = mi;
             }
-            R[2 + j] = make_float4(static_cast<float>(n[0]), static_cast<float>(n[1]), static_cast<float>(n[2]),
-                                   static_cast<float>(d));
+            face = make_float4(static_cast<float>(n[0]), static_cast<float>(n[1]), static_cast<float>(n[2]),
+                               static_cast<float>(d));
         }
     }
     if ((rc = gridUpload<float4>(ctx, &g.vRec, rec.data(), rec.size()))) return rc;

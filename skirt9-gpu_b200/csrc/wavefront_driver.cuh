@@ -166,10 +166,9 @@ cudaError_t runWave(const Wave& w, int numSMs, cudaStream_t s, unsigned long lon
     L.shadeBlocks = numSMs * (w.shadeBlocksPerSM > 0 ? w.shadeBlocksPerSM : 4);
     L.guideBlocks = numSMs * 2;
     L.guided = w.sc.guideMode == 2;
-    // the split traversal runs in captured graphs without per-stage timing, for walkers that gain
-    // from it
+    // the split traversal runs in captured graphs without per-stage timing
     L.split = false;
-    if (Walker::kSplit && useGraph && cache && (!timer || timer->level <= 1) && splitTraversal())
+    if (useGraph && cache && (!timer || timer->level <= 1) && splitTraversal())
     {
         if (cache->ensureSplit() == cudaSuccess)
         {
