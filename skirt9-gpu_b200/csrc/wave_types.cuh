@@ -22,7 +22,7 @@ struct alignas(128) PacketRec
     unsigned rngCtr;
     int rngHas;
     int nscatt, ellMix, ellRF;
-    int cell;   // cell of the last interaction (-1 after launch): start-cell hint of the next rays
+    int cell;   // cell of the launch position (-1: not searched) or of the last interaction: start cell of the next rays
     int scene;  // batched runs: the scene (simulation) of the slot's history
     int pad;
 };

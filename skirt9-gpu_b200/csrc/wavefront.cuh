@@ -908,7 +908,13 @@ static __global__ void launchPrepKernel(const __grid_constant__ Wave w, int nxt)
     for (int k = 0; k < NUM_KINDS; ++k) c->qn[1 - nxt][k] = 0;  // the buffer consumed by this pass
 }
 
-static __global__ void __launch_bounds__(256) launchKernel(const __grid_constant__ Wave w, int nxt)
+// The walkers that search for the cell of a start position (Walker::kLocates) take it from the packet:
+// it is found here once, for the packet's emission peel-offs and its first propagation rays alike
+// (five rays of the galaxy's packets, 26 % of all), and by full warps, where a traversal warp searches
+// for the few lanes that have just taken a task while the others wait. Only strictly inside the domain:
+// a start on its border is moved by the walker first.
+template<class Walker>
+__global__ void __launch_bounds__(256) launchKernel(const __grid_constant__ Wave w, int nxt)
 {
     int n = w.ctl->nLaunch;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
@@ -939,7 +945,14 @@ static __global__ void __launch_bounds__(256) launchKernel(const __grid_constant
         w.pk.rec[slot].ellMix = ell;
         w.pk.rec[slot].ellRF = sc.rfOn ? wlgBin(sc.rfB, sc.rfNb, sc.rfEll, o.lambda) : -1;
         if (w.anyStats) w.pk.nstat[slot] = 0;
-        w.pk.rec[slot].cell = -1;
+        int cell = -1;
+        if constexpr (Walker::kLocates)
+        {
+            const double* e = sc.g.ext;
+            if (o.x > e[0] && o.x < e[3] && o.y > e[1] && o.y < e[4] && o.z > e[2] && o.z < e[5] && o.L > 0)
+                cell = Walker::locate(sc.g, o.x, o.y, o.z);
+        }
+        w.pk.rec[slot].cell = cell;
         if (sc.guideMode == 2) w.pk.gRatio[slot] = 1.f;
         if (sc.guideMode == 1)
         {

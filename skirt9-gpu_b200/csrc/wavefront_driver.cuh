@@ -84,7 +84,7 @@ cudaError_t enqueuePass(const Wave& w, int pass, const WaveLaunch& L, cudaStream
     if (L.guided) guideScatterKernel<<<L.guideBlocks, GM_TILE, GM_SMEM_BYTES, s>>>(w, cur, nxt);
     if ((e = stageMark(t, pass, 6, s, capturing)) != cudaSuccess) return e;
     launchPrepKernel<<<1, 1, 0, s>>>(w, nxt);
-    launchKernel<<<L.shadeBlocks, L.threads, 0, s>>>(w, nxt);
+    launchKernel<Walker><<<L.shadeBlocks, L.threads, 0, s>>>(w, nxt);
     if ((e = stageMark(t, pass, 7, s, capturing)) != cudaSuccess) return e;
     return cudaGetLastError();
 }
