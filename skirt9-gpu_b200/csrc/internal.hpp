@@ -17,23 +17,21 @@ struct GraphCache
 {
     cudaGraphExec_t exec = nullptr;
     std::vector<unsigned char> key;
-    // the second stream and the events of the split traversal (peel-off rays and propagation rays
-    // walked by two kernels side by side), created with the first captured graph
+    // the second stream of the pipelined passes and its events, created with the first captured graph
     cudaStream_t side = nullptr;
-    cudaEvent_t fork = nullptr, peelDone = nullptr, join = nullptr;
-    bool lastSplit = false;  // the last run split its traversal (one more kernel per pass)
+    cudaEvent_t fork = nullptr, join = nullptr;
+    int kernelsPerPass = 0;  // of the last run
     void reset()
     {
         if (exec) cudaGraphExecDestroy(exec);
         exec = nullptr;
         key.clear();
     }
-    cudaError_t ensureSplit()
+    cudaError_t ensureSide()
     {
         cudaError_t e = cudaSuccess;
         if (!side) e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
         if (e == cudaSuccess && !fork) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
-        if (e == cudaSuccess && !peelDone) e = cudaEventCreateWithFlags(&peelDone, cudaEventDisableTiming);
         if (e == cudaSuccess && !join) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
         return e;
     }
@@ -41,10 +39,9 @@ struct GraphCache
     {
         reset();
         if (fork) cudaEventDestroy(fork);
-        if (peelDone) cudaEventDestroy(peelDone);
         if (join) cudaEventDestroy(join);
         if (side) cudaStreamDestroy(side);
-        fork = peelDone = join = nullptr;
+        fork = join = nullptr;
         side = nullptr;
     }
 };

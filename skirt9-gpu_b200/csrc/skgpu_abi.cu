@@ -206,7 +206,7 @@ int ensureWaveBuffers(skgpu_ctx* ctx, int P, int groups, int stats)
     int rc = 0;
     if ((rc = waveAlloc(ctx, &k.rec, P))) return rc;
     if ((rc = waveAlloc(ctx, &k.nstat, P))) return rc;
-    if ((rc = waveAlloc(ctx, &k.freeSlots, P))) return rc;
+    if ((rc = waveAlloc(ctx, &k.freeSlots, 2 * static_cast<size_t>(P)))) return rc;
     size_t ns = stats ? static_cast<size_t>(P) * STATS_CAP : 1;
     if ((rc = waveAlloc(ctx, &k.skey, ns))) return rc;
     if ((rc = waveAlloc(ctx, &k.sw, ns))) return rc;
@@ -231,6 +231,9 @@ int ensureWaveBuffers(skgpu_ctx* ctx, int P, int groups, int stats)
                 if ((rc = waveAlloc(ctx, &t.x, cap))) return rc;
                 if ((rc = waveAlloc(ctx, &t.y, cap))) return rc;
                 if ((rc = waveAlloc(ctx, &t.z, cap))) return rc;
+                if ((rc = waveAlloc(ctx, &t.lam, cap))) return rc;
+                if ((rc = waveAlloc(ctx, &t.ell, cap))) return rc;
+                if ((rc = waveAlloc(ctx, &t.cell, cap))) return rc;
             }
             if (kind == K_PEEL || kind == K_PROP1)
             {
@@ -1644,8 +1647,7 @@ static int runAndCollect(skgpu_ctx* ctx, const Wave& w, bool useGraph, bool time
     ctx->lastCounters.rf_stores = ctl.counters[4];
     ctx->lastCounters.stats_overflows = ctl.counters[5];
     ctx->lastCounters.stats_spilled = ctl.counters[6];
-    const int perPass = (w.sc.guideMode == 2 ? 8 : 7) + (useGraph && ctx->graphCache.lastSplit ? 1 : 0);
-    ctx->lastCounters.kernel_launches = static_cast<uint64_t>(passes) * perPass + 1 + (w.order ? 3 : 0);
+    ctx->lastCounters.kernel_launches = static_cast<uint64_t>(passes) * ctx->graphCache.kernelsPerPass + 1 + (w.order ? 3 : 0);
     ctx->lastPasses = passes;
     ctx->lastGuideWeightSum = ctl.guideWeightSum;
     ctx->lastGuideEvents = ctl.guideEvents;

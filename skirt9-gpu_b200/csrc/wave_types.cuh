@@ -50,7 +50,7 @@ struct PacketPool
     int* nstat;                // entries taken; above statCap the history has spilled
     StatSpill* spill;          // spill log of the run
     unsigned long long spillCap;
-    int* freeSlots;            // P
+    int* freeSlots;            // a stack of free slots (P), or with pipelined passes the slots freed by either parity (2 P)
     // pilot records of the guiding network: luminosity of the history detected by the target
     // instrument so far, last recorded event, event whose start value is still open
     double* gD;
@@ -66,6 +66,9 @@ struct TaskBuf
     int* info;      // PEEL: first instrument of the observer group | numScatt << 8
     double* par;    // PEEL: peel-off luminosity; PROP2/FREE: interaction optical depth
     double *x, *y, *z;  // PEEL: origin (the packet position at the event)
+    // PEEL, pipelined passes: what the ray needs of its packet, whose slot may by then hold another one
+    double* lam;      // wavelength
+    int *ell, *cell;  // dust-mix bin, start cell
     // results written by the trace kernel
     double* tau;    // PEEL / PROP1: optical depth (PROP1: of the complete path)
     int* m;         // PROP2 / FREE: interaction cell (-1: none)
@@ -76,8 +79,8 @@ struct TaskBuf
 struct Control
 {
     unsigned qn[2][NUM_KINDS];  // task counts per buffer and kind
-    unsigned traceCursor;   // next task of the pass (all kinds, or the peel-off kernel's)
-    unsigned traceCursor2;  // next propagation task of the pass (propagation kernel)
+    // next task of the pass: of all kinds or the peel-off kernel's, of the complete forced paths', of the searches'
+    unsigned traceCursor, forcedCursor, searchCursor;
     int freeTop;
     int nLaunch;
     int launchBase;
@@ -91,6 +94,9 @@ struct Control
     double guideWeightSum;           // guided scattering: sum of the weight factors (mean 1 in expectation)
     unsigned long long guideEvents;  // guided scattering events
     int err;
+    // pipelined passes: slots freed by either parity, and the blocks of a stage that have finished
+    int freeN[2];
+    unsigned peelTicket, stepTicket;
 };
 
 // Batched runs trace the histories of several independent scenes (simulations) through one
@@ -124,6 +130,7 @@ struct Wave
     unsigned long long first, count;
     int anyStats;
     int statCap;  // per-slot statistics buffer entries
+    int pipelined;  // the passes are the pipelined ones of a captured graph (wavefront_driver.cuh)
 };
 
 }  // namespace skg

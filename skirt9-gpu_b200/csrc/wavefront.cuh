@@ -195,14 +195,21 @@ SKG_D void guideCloseHistory(const Wave& w, int slot)
     }
 }
 
-SKG_D void endHistory(const Wave& w, int slot)
+SKG_D void endHistory(const Wave& w, int cur, int slot)
 {
     if (w.anyStats && w.pk.nstat[slot]) flushStats(w, slot);
     if (slotScene(w, slot).guideMode == 1) guideCloseHistory(w, slot);
-    int i = atomicAdd(&w.ctl->freeTop, 1);
-    w.pk.freeSlots[i] = slot;
+    if (w.pipelined)
+        w.pk.freeSlots[static_cast<size_t>(cur) * w.P + atomicAdd(&w.ctl->freeN[cur], 1)] = slot;
+    else
+        w.pk.freeSlots[atomicAdd(&w.ctl->freeTop, 1)] = slot;
     atomicAdd(&w.ctl->done, 1ULL);
 }
+
+// TaskBuf::info of a peel-off: the observer group's first instrument, the scene (batches), the number of
+// scattering events (for the scattering levels, of which there are far fewer than the cap)
+constexpr int PEEL_SCENE_SHIFT = 8, PEEL_SCATT_SHIFT = 14, PEEL_SCENE_MASK = (1 << (PEEL_SCATT_SHIFT - PEEL_SCENE_SHIFT)) - 1;
+static_assert(MAX_BATCH <= PEEL_SCENE_MASK + 1, "scene of a peel-off task");
 
 SKG_D void emitPeel(const Wave& w, int nxt, int slot, int group, int numScatt, double Lp, double x, double y,
                     double z)
@@ -210,11 +217,18 @@ SKG_D void emitPeel(const Wave& w, int nxt, int slot, int group, int numScatt, d
     const TaskBuf& b = w.q[nxt][K_PEEL];
     unsigned i = warpAppend(&w.ctl->qn[nxt][K_PEEL]);
     b.slot[i] = slot;
-    b.info[i] = group | (min(numScatt, (1 << 22)) << 8);
+    const PacketRec& p = w.pk.rec[slot];
+    b.info[i] = group | (w.nScenes > 1 ? p.scene << PEEL_SCENE_SHIFT : 0) | (min(numScatt, (1 << 17) - 1) << PEEL_SCATT_SHIFT);
     b.par[i] = Lp;
     b.x[i] = x;
     b.y[i] = y;
     b.z[i] = z;
+    if (w.pipelined)
+    {
+        b.lam[i] = p.lam;
+        b.ell[i] = p.ellMix;
+        b.cell[i] = p.cell;
+    }
 }
 
 SKG_D void emitProp(const Wave& w, int nxt, int kind, int slot, double par)
@@ -261,11 +275,11 @@ SKG_D float aadd(float a, float b) { return a + b; }
 SKG_D float amul(float a, float b) { return a * b; }
 SKG_D float aexp(float x) { return __expf(x); }
 
-// Mode selects the task kinds a launch walks: TRACE_ALL every kind; TRACE_PEEL the peel-off rays
-// and TRACE_PROP the propagation rays (PROP1, PROP2, FREE), two kernels that the captured pass graph
-// runs side by side on two streams, each with its own task cursor. The peel-off kernel, which walks
-// two thirds of the crossings of the galaxy, then carries none of the propagation tasks' state.
-enum TraceMode { TRACE_ALL = 0, TRACE_PEEL = 1, TRACE_PROP = 2 };
+// Mode selects the task kinds a launch walks: TRACE_ALL every kind, in one kernel; in the pipelined
+// passes TRACE_PEEL the peel-off rays, TRACE_FORCED the complete forced paths (PROP1) and TRACE_SEARCH
+// the interaction searches (PROP2, FREE), each with its own task cursor. A kernel of one kind carries
+// none of the others' state, and its lanes take the same branches.
+enum TraceMode { TRACE_ALL = 0, TRACE_PEEL = 1, TRACE_FORCED = 2, TRACE_SEARCH = 3 };
 
 template<class Walker, bool Multi = false, int Mode = TRACE_ALL>
 __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __grid_constant__ Wave w, int cur)
@@ -293,16 +307,21 @@ __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __g
     const int lane = threadIdx.x & 31;
     const int refillMin = w.refillMin > 0 ? w.refillMin : Walker::kRefillMin;
     unsigned n0 = w.ctl->qn[cur][0], n1 = w.ctl->qn[cur][1], n2 = w.ctl->qn[cur][2], n3 = w.ctl->qn[cur][3];
-    const unsigned total = Mode == TRACE_PEEL ? n0 : (Mode == TRACE_PROP ? n1 + n2 + n3 : n0 + n1 + n2 + n3);
+    const unsigned total = Mode == TRACE_PEEL ? n0 : Mode == TRACE_FORCED ? n1 : Mode == TRACE_SEARCH ? n2 + n3 : n0 + n1 + n2 + n3;
     if (total == 0) return;
-    unsigned* const cursor = Mode == TRACE_PROP ? &w.ctl->traceCursor2 : &w.ctl->traceCursor;
+    unsigned* const cursor = Mode == TRACE_FORCED   ? &w.ctl->forcedCursor
+                             : Mode == TRACE_SEARCH ? &w.ctl->searchCursor
+                                                    : &w.ctl->traceCursor;
 
     using Acc = typename Walker::Acc;  // FP64 (reference rounding) or FP32 optical depth and path length
     Walker wk;
-    int kind = -1;  // -1: needs a task, -2: finished
+    // -1: needs a task, -2: finished. A launch with fewer tasks than lanes spreads them over all its
+    // warps: the lanes of a warp then diverge less, which is what the time of a short queue depends on.
+    const unsigned warps = gridDim.x * (blockDim.x / 32);
+    int kind = static_cast<unsigned>(lane) < max(4u, (total + warps - 1) / warps) ? -1 : -2;
     // the task kind of a lane's current task, known at compile time where the mode fixes it
     auto isPeel = [&]() { return Mode == TRACE_PEEL || (Mode == TRACE_ALL && kind == K_PEEL); };
-    auto isProp1 = [&]() { return Mode != TRACE_PEEL && kind == K_PROP1; };
+    auto isProp1 = [&]() { return Mode == TRACE_FORCED || (Mode == TRACE_ALL && kind == K_PROP1); };
     unsigned idx = 0;
     int slot = 0;
     // Per-task accumulators. The task kinds never share a lane at the same time, so their
@@ -339,19 +358,20 @@ __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __g
                 }
                 else
                 {
-                    if (Mode == TRACE_PROP) t += n0;
-                    if (Mode == TRACE_PEEL || t < n0) { kind = K_PEEL; idx = t; }
-                    else if (t < n0 + n1) { kind = K_PROP1; idx = t - n0; }
+                    if (Mode == TRACE_FORCED) t += n0;
+                    if (Mode == TRACE_SEARCH) t += n0 + n1;
+                    if (Mode == TRACE_PEEL || (Mode == TRACE_ALL && t < n0)) { kind = K_PEEL; idx = t; }
+                    else if (Mode == TRACE_FORCED || (Mode == TRACE_ALL && t < n0 + n1)) { kind = K_PROP1; idx = t - n0; }
                     else if (t < n0 + n1 + n2) { kind = K_PROP2; idx = t - n0 - n1; }
                     else { kind = K_FREE; idx = t - n0 - n1 - n2; }
                     const TaskBuf& b = w.q[cur][kind];
                     slot = b.slot[idx];
-                    if constexpr (Multi) sid = w.pk.rec[slot].scene;
+                    if constexpr (Multi) sid = isPeel() ? (b.info[idx] >> PEEL_SCENE_SHIFT) & PEEL_SCENE_MASK : w.pk.rec[slot].scene;
                     // peel-off rays and complete forced paths (PROP1: radiation field) accumulate
                     // extinction; under explicit absorption the interaction searches (PROP2, FREE)
                     // walk on the scattering optical depth (setScatteringAndAbsorptionOpticalDepths)
                     {
-                        int ell = w.pk.rec[slot].ellMix;
+                        int ell = Mode == TRACE_PEEL ? b.ell[idx] : w.pk.rec[slot].ellMix;
                         sext = static_cast<Acc>(scn().explicitAbs && !isPeel() && kind >= K_PROP2 ? scn().mixSca[ell]
                                                                                                    : scn().mixExt[ell]);
                     }
@@ -363,7 +383,7 @@ __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __g
                         const InstrDev& in = scn().instr[b.info[idx] & 0xFF];
                         fA = static_cast<Acc>(log(b.par[idx]) + 745.);  // taumax = log(L) + 745
                         wk.start(scn().g, b.x[idx], b.y[idx], b.z[idx], in.kobs[0], in.kobs[1], in.kobs[2],
-                                 w.pk.rec[slot].cell);
+                                 Mode == TRACE_PEEL ? b.cell[idx] : w.pk.rec[slot].cell);
                     }
                     else
                     {
@@ -557,6 +577,16 @@ SKG_D void detectBin(const Wave& w, const Scene& sc, const InstrDev& in, int i, 
     }
 }
 
+// true in one thread of the block of a launch that finishes last
+SKG_D bool lastBlock(unsigned* ticket)
+{
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x != 0 || atomicAdd(ticket, 1u) + 1 != gridDim.x) return false;
+    __threadfence();
+    return true;
+}
+
 // FluxRecorder::detect for the instruments of one observer group (FluxRecorder.cpp:372-538)
 static __global__ void __launch_bounds__(256) shadePeelKernel(const __grid_constant__ Wave w, int cur)
 {
@@ -566,13 +596,14 @@ static __global__ void __launch_bounds__(256) shadePeelKernel(const __grid_const
     for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
     {
         int slot = b.slot[t];
-        const Scene& sc = slotScene(w, slot);
-        int group = b.info[t] & 0xFF;
-        int numScatt = b.info[t] >> 8;
+        const int info = b.info[t];
+        const Scene& sc = w.nScenes > 1 ? w.scenes[(info >> PEEL_SCENE_SHIFT) & PEEL_SCENE_MASK] : w.sc;
+        int group = info & 0xFF;
+        int numScatt = info >> PEEL_SCATT_SHIFT;
         double Lp = b.par[t];
         double ext = exp(-b.tau[t]);
         double x = b.x[t], y = b.y[t], z = b.z[t];
-        double lambda0 = w.pk.rec[slot].lam;
+        double lambda0 = w.pipelined ? b.lam[t] : w.pk.rec[slot].lam;
         for (int i = group; i < sc.ninstr && (i == group || sc.instr[i].same); ++i)
         {
             const InstrDev& in = sc.instr[i];
@@ -605,6 +636,12 @@ static __global__ void __launch_bounds__(256) shadePeelKernel(const __grid_const
         }
     }
     if (det) atomicAdd(&w.ctl->counters[3], det);
+    if (w.pipelined && lastBlock(&w.ctl->peelTicket))
+    {
+        w.ctl->qn[cur][K_PEEL] = 0;
+        w.ctl->traceCursor = 0;
+        w.ctl->peelTicket = 0;
+    }
 }
 
 // forced scattering: sample the interaction optical depth (simulateForcedPropagation)
@@ -629,7 +666,11 @@ static __global__ void __launch_bounds__(256) shadeProp1Kernel(const __grid_cons
         if (taupath <= 0.)
         {
             w.pk.rec[slot].L *= 0.;
-            endHistory(w, slot);
+            // in the pipelined passes the step ends the history (its detections may not be done yet)
+            if (w.pipelined)
+                emitProp(w, nxt, K_PROP2, slot, -1.);
+            else
+                endHistory(w, cur, slot);
             continue;
         }
         Rng rng;
@@ -694,7 +735,7 @@ SKG_D void interact(const Wave& w, int cur, int nxt, int slot, int m, double sIn
     if (m < 0)
     {
         atomicOr(&w.ctl->err, 2);  // MediumSystem::albedoForScattering: cannot locate the interaction point
-        endHistory(w, slot);
+        endHistory(w, cur, slot);
         return;
     }
     int ell = w.pk.rec[slot].ellMix;
@@ -737,7 +778,7 @@ SKG_D void interact(const Wave& w, int cur, int nxt, int slot, int m, double sIn
     if (sc.guideMode == 2 && w.pk.gRatio[slot] > 0.f) Lterm = L / static_cast<double>(w.pk.gRatio[slot]);
     if (L <= 0 || (forced && Lterm <= w.pk.rec[slot].Lth && nscatt >= sc.minScatt))
     {
-        endHistory(w, slot);
+        endHistory(w, cur, slot);
         return;
     }
     double g = sc.mixG[ell];
@@ -747,7 +788,7 @@ SKG_D void interact(const Wave& w, int cur, int nxt, int slot, int m, double sIn
     if (nscatt >= MAX_SCATT_EVENTS)
     {
         atomicOr(&w.ctl->err, 8);  // a history that never meets its termination criterion
-        endHistory(w, slot);
+        endHistory(w, cur, slot);
         return;
     }
     if (sc.guideMode == 2)
@@ -847,7 +888,7 @@ static __global__ void __launch_bounds__(GM_TILE) guideScatterKernel(const __gri
         if (!valid) continue;
         if (failed)
         {
-            endHistory(w, slot);  // the run reports the error; the history is not continued
+            endHistory(w, cur, slot);  // the run reports the error; the history is not continued
         }
         else
         {
@@ -884,7 +925,7 @@ static __global__ void __launch_bounds__(256) shadeFreeKernel(const __grid_const
     for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
     {
         if (!b.found[t])
-            endHistory(w, b.slot[t]);  // the interaction point is outside the path: the packet escapes
+            endHistory(w, cur, b.slot[t]);  // the interaction point is outside the path: the packet escapes
         else
             interact(w, cur, nxt, b.slot[t], b.m[t], b.s[t], false, b.par[t]);
     }
@@ -904,22 +945,22 @@ static __global__ void launchPrepKernel(const __grid_constant__ Wave w, int nxt)
     c->launchHist0 = w.first + c->launched;
     c->launched += n;
     c->traceCursor = 0;
-    c->traceCursor2 = 0;
     for (int k = 0; k < NUM_KINDS; ++k) c->qn[1 - nxt][k] = 0;  // the buffer consumed by this pass
 }
 
+// New histories in the nLaunch free slots of the list.
 // The walkers that search for the cell of a start position (Walker::kLocates) take it from the packet:
 // it is found here once, for the packet's emission peel-offs and its first propagation rays alike
 // (five rays of the galaxy's packets, 26 % of all), and by full warps, where a traversal warp searches
 // for the few lanes that have just taken a task while the others wait. Only strictly inside the domain:
 // a start on its border is moved by the walker first.
 template<class Walker>
-__global__ void __launch_bounds__(256) launchKernel(const __grid_constant__ Wave w, int nxt)
+SKG_D void launchHistories(const Wave& w, int nxt, const int* slots)
 {
-    int n = w.ctl->nLaunch;
+    const int n = w.ctl->nLaunch;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
     {
-        int slot = w.pk.freeSlots[w.ctl->launchBase + t];
+        int slot = slots[t];
         unsigned long long hist = w.ctl->launchHist0 + t;
         if (w.order) hist = w.first + w.order[hist - w.first];  // wavelength-ordered launch
         if (w.nScenes > 1)
@@ -964,7 +1005,7 @@ __global__ void __launch_bounds__(256) launchKernel(const __grid_constant__ Wave
         if (!(o.L > 0))
         {
             storeRng(w, slot, rng);
-            endHistory(w, slot);
+            endHistory(w, 1 - nxt, slot);
             continue;
         }
         if (sc.peel && sc.ninstr > 0) emitPeels(w, nxt, slot, false, 0, o.L, 0., o.x, o.y, o.z, 0., 0., 0.);
@@ -973,11 +1014,62 @@ __global__ void __launch_bounds__(256) launchKernel(const __grid_constant__ Wave
     }
 }
 
+template<class Walker>
+__global__ void __launch_bounds__(256) launchKernel(const __grid_constant__ Wave w, int nxt)
+{
+    launchHistories<Walker>(w, nxt, w.pk.freeSlots + w.ctl->launchBase);
+}
+
+// end of a pipelined pass: the queues that it consumed are empty, and the slots that it freed are the
+// next step's to launch into
+SKG_D void closePass(const Wave& w, int cur)
+{
+    volatile Control* c = w.ctl;  // freeN was counted by other blocks of this launch
+    const unsigned long long launched = c->launched;
+    const int n = static_cast<int>(min(static_cast<unsigned long long>(c->freeN[cur]), w.count - launched));
+    c->nLaunch = n;
+    c->launchHist0 = w.first + launched;
+    c->launched = launched + n;
+    c->freeN[1 - cur] = 0;
+    c->qn[cur][K_PROP1] = 0;
+    c->qn[cur][K_PROP2] = 0;
+    c->qn[cur][K_FREE] = 0;
+    c->qn[cur][K_GUIDE] = 0;
+    c->forcedCursor = 0;
+    c->searchCursor = 0;
+    c->stepTicket = 0;
+}
+
+// The step between two pipelined traversals: the interactions at the ends of the searches, and new
+// histories in the slots that the previous step freed (so that one launch does both). The block that
+// finishes last closes the pass, unless a guided-scattering stage follows.
+template<class Walker>
+__global__ void __launch_bounds__(256) stepKernel(const __grid_constant__ Wave w, int cur, int nxt, int close)
+{
+    const unsigned n2 = w.ctl->qn[cur][K_PROP2], n3 = w.ctl->qn[cur][K_FREE];
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n2 + n3; t += gridDim.x * blockDim.x)
+    {
+        const bool forced = t < n2;
+        const TaskBuf& b = w.q[cur][forced ? K_PROP2 : K_FREE];
+        const unsigned i = forced ? t : t - n2;
+        // an empty forced path ends its history, and a free one whose interaction point is outside: the
+        // packet escapes
+        if (forced ? b.par[i] < 0. : !b.found[i])
+            endHistory(w, cur, b.slot[i]);
+        else
+            interact(w, cur, nxt, b.slot[i], b.m[i], b.s[i], forced, b.par[i]);
+    }
+    launchHistories<Walker>(w, nxt, w.pk.freeSlots + static_cast<size_t>(nxt) * w.P);
+    if (close && lastBlock(&w.ctl->stepTicket)) closePass(w, cur);
+}
+
+static __global__ void closePassKernel(const __grid_constant__ Wave w, int cur) { closePass(w, cur); }
+
 static __global__ void initPoolKernel(const __grid_constant__ Wave w)
 {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < w.P; t += gridDim.x * blockDim.x)
     {
-        w.pk.freeSlots[t] = t;
+        w.pk.freeSlots[w.pipelined ? static_cast<size_t>(w.P) + t : t] = t;
         if (w.anyStats)
         {
             w.pk.nstat[t] = 0;
@@ -990,13 +1082,15 @@ static __global__ void initPoolKernel(const __grid_constant__ Wave w)
         for (int b = 0; b < 2; ++b)
             for (int k = 0; k < NUM_KINDS; ++k) c->qn[b][k] = 0;
         c->traceCursor = 0;
-        c->traceCursor2 = 0;
+        c->forcedCursor = c->searchCursor = 0;
         c->freeTop = w.P;
-        c->nLaunch = 0;
+        c->nLaunch = w.pipelined ? static_cast<int>(min(static_cast<unsigned long long>(w.P), w.count)) : 0;
         c->launchBase = 0;
-        c->launched = 0;
+        c->launched = c->nLaunch;
         c->done = 0;
-        c->launchHist0 = 0;
+        c->launchHist0 = w.pipelined ? w.first : 0;
+        c->freeN[0] = c->freeN[1] = 0;
+        c->peelTicket = c->stepTicket = 0;
         for (int k = 0; k < 8; ++k) c->counters[k] = 0;
         c->spillN = 0;
         c->guideWeightSum = 0.;

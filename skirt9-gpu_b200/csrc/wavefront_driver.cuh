@@ -17,11 +17,12 @@ struct WaveLaunch
 {
     int traceBlocks, shadeBlocks, guideBlocks, threads;
     bool guided, multi;
-    // split traversal: the peel-off kernel on the side stream, the propagation kernel on the main one
-    bool split;
-    int peelBlocks, propBlocks;
+    // pipelined passes: whether detections come before the step that may end their history, whether
+    // any scene forces its scattering, and the second stream with its events
+    bool pipelined, strict, forced;
+    int peelBlocks, forcedBlocks, searchBlocks;
     cudaStream_t side;
-    cudaEvent_t fork, peelDone, join;
+    cudaEvent_t fork, join;
 };
 
 // shared memory of the traversal kernel: the scene table of a batch
@@ -46,34 +47,57 @@ void launchTrace(const Wave& w, int cur, int blocks, const WaveLaunch& L, cudaSt
         traceKernel<Walker, false, Mode><<<blocks, L.threads, 0, s>>>(w, cur);
 }
 
-// `pass` is the index of the pass within its batch (selects the timer's events)
+// The passes of a captured graph without stage timing, on two streams:
+//   main  traversal of the complete forced paths, sampling of their interaction depths, traversal of
+//         the searches for the interaction points, then the step (interactions, new histories)
+//   side  traversal of the peel-off rays that the previous step queued, then their detection
+// One pass carries a packet from one interaction to the next. A peel-off task holds what it needs of
+// its packet, so the packet goes on meanwhile: the side stream may lag by a pass, and the last long
+// rays of one traversal run beside the next one instead of alone. Only where the statistics or the
+// pilot records of a history are closed at its end do its detections come first (`strict`).
+// The plain pass below walks the forced paths and the searches in passes of their own (twice the
+// passes, each as long as its longest ray), joins its streams in each, and takes eight kernels.
+template<class Walker>
+cudaError_t enqueuePipelined(const Wave& w, int pass, const WaveLaunch& L, cudaStream_t s)
+{
+    const int cur = pass & 1, nxt = 1 - cur;
+    cudaError_t e;
+    if ((e = cudaEventRecord(L.fork, s)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(L.side, L.fork, 0)) != cudaSuccess) return e;
+    if (L.forced)
+    {
+        launchTrace<Walker, TRACE_FORCED>(w, cur, L.forcedBlocks, L, s);
+        shadeProp1Kernel<<<L.shadeBlocks, L.threads, 0, s>>>(w, cur, cur);
+    }
+    launchTrace<Walker, TRACE_SEARCH>(w, cur, L.searchBlocks, L, s);
+    // the step refills the peel-off queue that the side stream emptied in the previous pass
+    if (!L.strict && pass > 0 && (e = cudaStreamWaitEvent(s, L.join, 0)) != cudaSuccess) return e;
+    launchTrace<Walker, TRACE_PEEL>(w, cur, L.peelBlocks, L, L.side);
+    shadePeelKernel<<<L.shadeBlocks, L.threads, 0, L.side>>>(w, cur);
+    if ((e = cudaEventRecord(L.join, L.side)) != cudaSuccess) return e;
+    if (L.strict && (e = cudaStreamWaitEvent(s, L.join, 0)) != cudaSuccess) return e;
+    stepKernel<Walker><<<L.shadeBlocks, L.threads, 0, s>>>(w, cur, nxt, L.guided ? 0 : 1);
+    if (L.guided)
+    {
+        guideScatterKernel<<<L.guideBlocks, GM_TILE, GM_SMEM_BYTES, s>>>(w, cur, nxt);
+        closePassKernel<<<1, 1, 0, s>>>(w, cur);
+    }
+    // the last pass of a graph ends with both streams
+    if (pass + 1 == StageTimer::kBatch && (e = cudaStreamWaitEvent(s, L.join, 0)) != cudaSuccess) return e;
+    return cudaGetLastError();
+}
+
+// A plain pass, for stage timing and for runs without graphs. `pass` is the index of the pass within
+// its batch (selects the timer's events).
 template<class Walker>
 cudaError_t enqueuePass(const Wave& w, int pass, const WaveLaunch& L, cudaStream_t s, StageTimer* t, bool capturing)
 {
     int cur = pass & 1, nxt = 1 - cur;
     cudaError_t e;
     if ((e = stageMark(t, pass, 0, s, capturing)) != cudaSuccess) return e;
-    if (L.split)
-    {
-        // peel-off rays and their detection on the side stream, propagation rays on this one; the
-        // stage kernels that end histories (and flush their statistics) wait for the detection
-        if ((e = cudaEventRecord(L.fork, s)) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(L.side, L.fork, 0)) != cudaSuccess) return e;
-        launchTrace<Walker, TRACE_PEEL>(w, cur, L.peelBlocks, L, L.side);
-        if ((e = cudaEventRecord(L.peelDone, L.side)) != cudaSuccess) return e;
-        shadePeelKernel<<<L.shadeBlocks, L.threads, 0, L.side>>>(w, cur);
-        if ((e = cudaEventRecord(L.join, L.side)) != cudaSuccess) return e;
-        launchTrace<Walker, TRACE_PROP>(w, cur, L.propBlocks, L, s);
-        if ((e = cudaStreamWaitEvent(s, L.peelDone, 0)) != cudaSuccess) return e;
-        if ((e = stageMark(t, pass, 1, s, capturing)) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(s, L.join, 0)) != cudaSuccess) return e;
-    }
-    else
-    {
-        launchTrace<Walker, TRACE_ALL>(w, cur, L.traceBlocks, L, s);
-        if ((e = stageMark(t, pass, 1, s, capturing)) != cudaSuccess) return e;
-        shadePeelKernel<<<L.shadeBlocks, L.threads, 0, s>>>(w, cur);
-    }
+    launchTrace<Walker, TRACE_ALL>(w, cur, L.traceBlocks, L, s);
+    if ((e = stageMark(t, pass, 1, s, capturing)) != cudaSuccess) return e;
+    shadePeelKernel<<<L.shadeBlocks, L.threads, 0, s>>>(w, cur);
     if ((e = stageMark(t, pass, 2, s, capturing)) != cudaSuccess) return e;
     shadeProp1Kernel<<<L.shadeBlocks, L.threads, 0, s>>>(w, cur, nxt);
     if ((e = stageMark(t, pass, 3, s, capturing)) != cudaSuccess) return e;
@@ -96,8 +120,8 @@ cudaError_t enqueuePass(const Wave& w, int pass, const WaveLaunch& L, cudaStream
 // pass limit is reached without finishing. `passes` receives the number of passes run.
 // the inputs a captured pass graph depends on: the wave parameters (by value in every kernel
 // node), the launch shape, the walker and the timing events recorded into it
-// the split traversal is on unless SKGPU_SPLIT_TRAVERSAL=0 (a switch for comparing the two forms)
-inline bool splitTraversal()
+// the pipelined passes are on unless SKGPU_SPLIT_TRAVERSAL=0 (a switch for comparing the two forms)
+inline bool pipelinedPasses()
 {
     static const bool on = [] {
         const char* v = std::getenv("SKGPU_SPLIT_TRAVERSAL");
@@ -128,10 +152,12 @@ void applyTraceCarveout()
     auto set = [pct](const void* f) { cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, pct); };
     set(reinterpret_cast<const void*>(&traceKernel<Walker, false, TRACE_ALL>));
     set(reinterpret_cast<const void*>(&traceKernel<Walker, false, TRACE_PEEL>));
-    set(reinterpret_cast<const void*>(&traceKernel<Walker, false, TRACE_PROP>));
+    set(reinterpret_cast<const void*>(&traceKernel<Walker, false, TRACE_FORCED>));
+    set(reinterpret_cast<const void*>(&traceKernel<Walker, false, TRACE_SEARCH>));
     set(reinterpret_cast<const void*>(&traceKernel<Walker, true, TRACE_ALL>));
     set(reinterpret_cast<const void*>(&traceKernel<Walker, true, TRACE_PEEL>));
-    set(reinterpret_cast<const void*>(&traceKernel<Walker, true, TRACE_PROP>));
+    set(reinterpret_cast<const void*>(&traceKernel<Walker, true, TRACE_FORCED>));
+    set(reinterpret_cast<const void*>(&traceKernel<Walker, true, TRACE_SEARCH>));
 }
 
 template<class Walker>
@@ -153,9 +179,10 @@ std::vector<unsigned char> graphKey(const Wave& w, const WaveLaunch& L, const St
 }
 
 template<class Walker>
-cudaError_t runWave(const Wave& w, int numSMs, cudaStream_t s, unsigned long long* doneHost, long long* passes,
+cudaError_t runWave(const Wave& wave, int numSMs, cudaStream_t s, unsigned long long* doneHost, long long* passes,
                     long long maxPasses, bool useGraph, StageTimer* timer, GraphCache* cache = nullptr)
 {
+    Wave w = wave;
     WaveLaunch L{};
     L.threads = 256;
     applyTraceCarveout<Walker>();
@@ -166,21 +193,20 @@ cudaError_t runWave(const Wave& w, int numSMs, cudaStream_t s, unsigned long lon
     L.shadeBlocks = numSMs * (w.shadeBlocksPerSM > 0 ? w.shadeBlocksPerSM : 4);
     L.guideBlocks = numSMs * 2;
     L.guided = w.sc.guideMode == 2;
-    // the split traversal runs in captured graphs without per-stage timing
-    L.split = false;
-    if (useGraph && cache && (!timer || timer->level <= 1) && splitTraversal())
+    if (useGraph && cache && !timer && pipelinedPasses() && cache->ensureSide() == cudaSuccess)
     {
-        if (cache->ensureSplit() == cudaSuccess)
-        {
-            L.split = true;
-            int cap = w.traceBlocksPerSM > 0 ? w.traceBlocksPerSM : 1 << 30;
-            L.peelBlocks = numSMs * std::min(cap, traceBlocksPerSM<Walker, TRACE_PEEL>(L.multi, traceSmemBytes(w)));
-            L.propBlocks = numSMs * std::min(cap, traceBlocksPerSM<Walker, TRACE_PROP>(L.multi, traceSmemBytes(w)));
-            L.side = cache->side;
-            L.fork = cache->fork;
-            L.peelDone = cache->peelDone;
-            L.join = cache->join;
-        }
+        L.pipelined = true;
+        L.strict = w.anyStats || w.sc.guideMode == 1;
+        L.forced = w.nScenes > 1 || w.sc.forced;
+        const int cap = w.traceBlocksPerSM > 0 ? w.traceBlocksPerSM : 1 << 30;
+        const size_t smem = traceSmemBytes(w);
+        L.peelBlocks = numSMs * std::min(cap, traceBlocksPerSM<Walker, TRACE_PEEL>(L.multi, smem));
+        L.forcedBlocks = numSMs * std::min(cap, traceBlocksPerSM<Walker, TRACE_FORCED>(L.multi, smem));
+        L.searchBlocks = numSMs * std::min(cap, traceBlocksPerSM<Walker, TRACE_SEARCH>(L.multi, smem));
+        L.side = cache->side;
+        L.fork = cache->fork;
+        L.join = cache->join;
+        w.pipelined = 1;
     }
     *passes = 0;
     if (timer)
@@ -190,7 +216,7 @@ cudaError_t runWave(const Wave& w, int numSMs, cudaStream_t s, unsigned long lon
         cudaError_t ea = cudaFuncSetAttribute(guideScatterKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GM_SMEM_BYTES);
         if (ea != cudaSuccess) return ea;
     }
-    if (cache) cache->lastSplit = L.split;
+    if (cache) cache->kernelsPerPass = (L.pipelined ? (L.forced ? 6 : 4) + (L.guided ? 1 : 0) : 7) + (L.guided ? 1 : 0);
     initPoolKernel<<<L.shadeBlocks, L.threads, 0, s>>>(w);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -213,7 +239,8 @@ cudaError_t runWave(const Wave& w, int numSMs, cudaStream_t s, unsigned long lon
     {
         e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
-        for (int k = 0; k < passesPerBatch && e == cudaSuccess; ++k) e = enqueuePass<Walker>(w, k, L, s, timer, true);
+        for (int k = 0; k < passesPerBatch && e == cudaSuccess; ++k)
+            e = L.pipelined ? enqueuePipelined<Walker>(w, k, L, s) : enqueuePass<Walker>(w, k, L, s, timer, true);
         cudaError_t e2 = cudaStreamEndCapture(s, &graph);
         if (e == cudaSuccess) e = e2;
         if (e != cudaSuccess)
