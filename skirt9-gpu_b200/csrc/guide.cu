@@ -15,10 +15,8 @@ namespace skg {
 namespace {
 
 // ---------------------------------------------------------------------------------------------
-// FP32 forward / backward of one sample (training and gradient checks)
+// FP32 forward pass of one sample: raw outputs and the activations of the hidden layers
 // ---------------------------------------------------------------------------------------------
-
-// raw outputs and the activations of the hidden layers
 SKG_D void mlpForward(const float* P, const float* in, float* h /*4 x 64*/, float* out)
 {
     const float* cur = in;
@@ -39,117 +37,198 @@ SKG_D void mlpForward(const float* P, const float* in, float* h /*4 x 64*/, floa
     }
 }
 
-// log q(k) of the mixture and its gradient with respect to the 40 raw outputs
-SKG_D float headLogDensityGrad(const float* o, const float* k, float* g)
+// ---------------------------------------------------------------------------------------------
+// Loss and gradient of a batch, in FP32 on the CUDA cores (the training keeps 32 bits throughout).
+//
+// One block per SM takes its share of the batch in tiles of S samples and keeps everything of a tile
+// on chip: the network (67 KB) and the activations of all layers in shared memory, the sums of the
+// weight gradients in registers (a thread holds a 4 x 4 patch of every layer's matrix) until its last
+// tile. Forward pass, back-propagation and weight gradients are all products of a 64-wide and an
+// S-wide side, computed as 4 x S/16 patches per thread from float4 reads; rows are padded to 68 floats
+// so that the reads of a warp fall on different banks. The blocks' sums go to `partial` and
+// gradSumKernel adds them, in block order: the result does not depend on timing.
+//
+// 12 wavefronts of shared memory per 64 multiply-adds of a warp, so the multiply-adds bound it: 1.5
+// GFLOP for 16 384 samples. One thread per sample with its activations in local memory, and one thread
+// per parameter that went over the whole batch, took 1.9 ms for them, copies and all 2.05 ms; now the
+// call takes 0.21 ms (B200), most of it the copies of its host arrays.
+// ---------------------------------------------------------------------------------------------
+constexpr int GB_THREADS = 256;
+constexpr int GB_LD = 68, GB_LD0 = 12;  // row lengths in floats: 64-wide rows, and the 8 inputs
+// row-padded weights of layer l in shared memory, then the biases
+SKG_HD constexpr int gbW(int l) { return l == 0 ? 0 : 64 * GB_LD0 + (l - 1) * 64 * GB_LD; }
+constexpr int GB_B = 64 * GB_LD0 + 3 * 64 * GB_LD + GUIDE_OUT * GB_LD;
+constexpr int GB_X = GB_B + 4 * 64 + GUIDE_OUT;  // activations: inputs, 4 hidden layers, 2 delta buffers
+constexpr int gbFloats(int S) { return GB_X + S * GB_LD0 + 6 * S * GB_LD + 4 * S; }
+constexpr int GB_PARTIAL = GUIDE_NPARAMS + 1;  // per block: the gradient and the loss
+
+SKG_D float dot4(float4 a, float4 b, float acc)
 {
-    GuideMixture m;
-    guideMixture(o, m);
-    float l[GUIDE_LOBES], cs[GUIDE_LOBES];
-    float lmax = -INFINITY;
-    for (int j = 0; j < GUIDE_LOBES; ++j)
+    return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
+}
+SKG_D float4 axpy4(float a, float4 x, float4 y)
+{
+    return make_float4(fmaf(a, x.x, y.x), fmaf(a, x.y, y.y), fmaf(a, x.z, y.z), fmaf(a, x.w, y.w));
+}
+SKG_D float4 row4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// Y[s][o] = act(b[o] + sum_i W[o][i] X[s][i]) for the S samples of a tile
+template<int S, int K, int LD, int N, bool Relu>
+SKG_D void tileForward(const float* W, const float* b, const float* X, float* Y)
+{
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    constexpr int SJ = S / 16, OJ = (N + 15) / 16;
+    float acc[SJ][OJ];
+#pragma unroll
+    for (int j = 0; j < OJ; ++j)
+#pragma unroll
+        for (int i = 0; i < SJ; ++i) acc[i][j] = tx + 16 * j < N ? b[tx + 16 * j] : 0.f;
+#pragma unroll 4
+    for (int k = 0; k < K; k += 4)
     {
-        cs[j] = m.mu[j][0] * k[0] + m.mu[j][1] * k[1] + m.mu[j][2] * k[2];
-        l[j] = m.logw[j] + logVmf(m.kappa[j], cs[j]);
+        float4 w[OJ], x[SJ];
+#pragma unroll
+        for (int j = 0; j < OJ; ++j) w[j] = row4(W + min(tx + 16 * j, N - 1) * LD + k);
+#pragma unroll
+        for (int i = 0; i < SJ; ++i) x[i] = row4(X + (ty + 16 * i) * LD + k);
+#pragma unroll
+        for (int i = 0; i < SJ; ++i)
+#pragma unroll
+            for (int j = 0; j < OJ; ++j) acc[i][j] = dot4(w[j], x[i], acc[i][j]);
+    }
+#pragma unroll
+    for (int i = 0; i < SJ; ++i)
+#pragma unroll
+        for (int j = 0; j < OJ; ++j)
+            if (tx + 16 * j < N) Y[(ty + 16 * i) * GB_LD + tx + 16 * j] = Relu ? fmaxf(acc[i][j], 0.f) : acc[i][j];
+}
+
+// P[s][i] = (sum_o W[o][i] D[s][o]) where the activation H[s][i] is positive, else 0
+template<int S, int N>
+SKG_D void tileBackward(const float* W, const float* D, const float* H, float* P)
+{
+    const int i0 = 4 * (threadIdx.x & 15), ty = threadIdx.x >> 4;
+    constexpr int SJ = S / 16;
+    float4 acc[SJ];
+#pragma unroll
+    for (int i = 0; i < SJ; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+    for (int o = 0; o < N; o += 4)
+    {
+        const float4 w0 = row4(W + o * GB_LD + i0), w1 = row4(W + (o + 1) * GB_LD + i0), w2 = row4(W + (o + 2) * GB_LD + i0),
+                     w3 = row4(W + (o + 3) * GB_LD + i0);
+#pragma unroll
+        for (int i = 0; i < SJ; ++i)
+        {
+            const float4 d = row4(D + (ty + 16 * i) * GB_LD + o);
+            acc[i] = axpy4(d.w, w3, axpy4(d.z, w2, axpy4(d.y, w1, axpy4(d.x, w0, acc[i]))));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < SJ; ++i)
+    {
+        const float4 h = row4(H + (ty + 16 * i) * GB_LD + i0);
+        *reinterpret_cast<float4*>(P + (ty + 16 * i) * GB_LD + i0) =
+            make_float4(h.x > 0.f ? acc[i].x : 0.f, h.y > 0.f ? acc[i].y : 0.f, h.z > 0.f ? acc[i].z : 0.f,
+                        h.w > 0.f ? acc[i].w : 0.f);
+    }
+}
+
+// G[r] += sum_s D[s][4 ty + r] H[s][4 tx ...] over the tile (rows of the weight gradient)
+template<int S>
+SKG_D void tileWeights(const float* D, const float* H, float4* G)
+{
+    const int i0 = 4 * (threadIdx.x & 15), o0 = 4 * (threadIdx.x >> 4);
+#pragma unroll 4
+    for (int s = 0; s < S; ++s)
+    {
+        const float4 d = row4(D + s * GB_LD + o0), h = row4(H + s * GB_LD + i0);
+        G[0] = axpy4(d.x, h, G[0]);
+        G[1] = axpy4(d.y, h, G[1]);
+        G[2] = axpy4(d.z, h, G[2]);
+        G[3] = axpy4(d.w, h, G[3]);
+    }
+}
+
+// the part of a bias gradient of N outputs that a quarter of the block's threads sums: thread t the
+// output t % 64 over every fourth sample from t / 64 on
+template<int S>
+SKG_D float tileBias(const float* D, int N)
+{
+    const int o = threadIdx.x & 63;
+    float acc = 0.f;
+    if (o < N)
+        for (int s = threadIdx.x >> 6; s < S; s += 4) acc += D[s * GB_LD + o];
+    return acc;
+}
+
+// Log density of the mixture of a sample's outputs `o` at the direction k, and the deltas of the
+// outputs for the loss -w log q: GS neighbouring lanes share a sample, each with 8 / GS lobes. Returns
+// the sample's loss in the first of them, 0 in the others.
+template<int S>
+SKG_D float tileHead(const float* o, const float* k, float w, bool valid, float* dout)
+{
+    constexpr int GS = GB_THREADS / S, J = GUIDE_LOBES / GS;
+    const int q = threadIdx.x % GS;
+    auto over = [](float v, bool mx) {
+#pragma unroll
+        for (int m = 1; m < GS; m <<= 1)
+        {
+            const float u = __shfl_xor_sync(0xffffffffu, v, m);
+            v = mx ? fmaxf(v, u) : v + u;
+        }
+        return v;
+    };
+    float amax = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < J; ++j) amax = fmaxf(amax, o[5 * (q * J + j)]);
+    amax = over(amax, true);
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < J; ++j) sum += expf(o[5 * (q * J + j)] - amax);
+    const float lse = amax + logf(over(sum, false));
+    float logw[J], l[J], cs[J], kap[J], mu[J][3], len[J];
+    float lmax = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+    {
+        const float* r = o + 5 * (q * J + j);
+        logw[j] = r[0] - lse;
+        len[j] = sqrtf(r[1] * r[1] + r[2] * r[2] + r[3] * r[3]);
+        const bool ok = len[j] > 1e-12f;
+        mu[j][0] = ok ? r[1] / len[j] : 0.f;
+        mu[j][1] = ok ? r[2] / len[j] : 0.f;
+        mu[j][2] = ok ? r[3] / len[j] : 1.f;
+        kap[j] = fminf(softplusf(r[4]) + GUIDE_KAPPA_MIN, GUIDE_KAPPA_MAX);
+        cs[j] = mu[j][0] * k[0] + mu[j][1] * k[1] + mu[j][2] * k[2];
+        l[j] = logw[j] + logVmf(kap[j], cs[j]);
         lmax = fmaxf(lmax, l[j]);
     }
-    float s = 0.f;
-    for (int j = 0; j < GUIDE_LOBES; ++j) s += expf(l[j] - lmax);
-    float logq = lmax + logf(s);
-    for (int j = 0; j < GUIDE_LOBES; ++j)
+    lmax = over(lmax, true);
+    sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < J; ++j) sum += expf(l[j] - lmax);
+    const float logq = lmax + logf(over(sum, false));
+#pragma unroll
+    for (int j = 0; j < J; ++j)
     {
-        float r = expf(l[j] - logq);   // responsibility
-        float w = expf(m.logw[j]);     // mixture weight
-        g[5 * j] = r - w;
+        const float r = expf(l[j] - logq);  // responsibility
+        float g[5];
+        g[0] = r - expf(logw[j]);
         // direction: mu = a / |a|, d log f / d a = kappa (k - (mu.k) mu) / |a|
-        float a0 = o[5 * j + 1], a1 = o[5 * j + 2], a2 = o[5 * j + 3];
-        float n = sqrtf(a0 * a0 + a1 * a1 + a2 * a2);
-        if (n > 1e-12f)
-        {
-            float c = r * m.kappa[j] / n;
-            g[5 * j + 1] = c * (k[0] - cs[j] * m.mu[j][0]);
-            g[5 * j + 2] = c * (k[1] - cs[j] * m.mu[j][1]);
-            g[5 * j + 3] = c * (k[2] - cs[j] * m.mu[j][2]);
-        }
-        else
-        {
-            g[5 * j + 1] = g[5 * j + 2] = g[5 * j + 3] = 0.f;
-        }
+        const float c = len[j] > 1e-12f ? r * kap[j] / len[j] : 0.f;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) g[1 + a] = c != 0.f ? c * (k[a] - cs[j] * mu[j][a]) : 0.f;
         // concentration: kappa = softplus(s) + kmin, clamped at kmax
-        float kap = m.kappa[j];
-        float e = expf(-2.f * kap);
-        float dlogf = 1.f / kap - 2.f * e / (1.f - e) + (cs[j] - 1.f);
-        float sraw = o[5 * j + 4];
-        float dk = (softplusf(sraw) + GUIDE_KAPPA_MIN < GUIDE_KAPPA_MAX) ? 1.f / (1.f + expf(-sraw)) : 0.f;
-        g[5 * j + 4] = r * dlogf * dk;
+        const float e = expf(-2.f * kap[j]);
+        const float dlogf = 1.f / kap[j] - 2.f * e / (1.f - e) + (cs[j] - 1.f);
+        const float sraw = o[5 * (q * J + j) + 4];
+        const float dk = (softplusf(sraw) + GUIDE_KAPPA_MIN < GUIDE_KAPPA_MAX) ? 1.f / (1.f + expf(-sraw)) : 0.f;
+        g[4] = r * dlogf * dk;
+#pragma unroll
+        for (int a = 0; a < 5; ++a) dout[5 * (q * J + j) + a] = valid ? -w * g[a] : 0.f;
     }
-    return logq;
-}
-
-// Per-sample pass of a batch: forward, loss -w log q, and the back-propagated deltas. Writes, per
-// sample b, the inputs (8), hidden activations (4 x 64) and the deltas of every layer's
-// pre-activation (4 x 64 hidden, 40 output) to the scratch rows used by the weight-gradient kernel.
-struct BatchScratch
-{
-    float* in;     // B x 8
-    float* h;      // B x 256
-    float* delta;  // B x 296 (hidden 4 x 64, then 40)
-    float* loss;   // 1 (accumulated)
-};
-
-constexpr int DELTA_W = 4 * 64 + GUIDE_OUT;
-
-SKG_D void samplePass(const float* P, const float* in, const float* k, float w, const BatchScratch& s, int b,
-                      float& lossOut)
-{
-    float h[4 * 64], out[GUIDE_OUT], g[GUIDE_OUT];
-    mlpForward(P, in, h, out);
-    float logq = headLogDensityGrad(out, k, g);
-    lossOut = -w * logq;
-    float* d = s.delta + static_cast<size_t>(b) * DELTA_W;
-    // loss = -w log q: delta of the outputs
-    float dout[GUIDE_OUT];
-    for (int o = 0; o < GUIDE_OUT; ++o)
-    {
-        dout[o] = -w * g[o];
-        d[256 + o] = dout[o];
-    }
-    // back through the hidden layers: delta_l = (W_{l+1}^T delta_{l+1}) * relu'(h_l)
-    float nextDelta[64];
-    const float* dn = dout;
-    int nOut = GUIDE_OUT;
-    for (int l = GUIDE_LAYERS - 2; l >= 0; --l)
-    {
-        const float* W = P + guideParamOffset(l + 1);  // (nOut x 64)
-        float cur[64];
-        for (int i = 0; i < 64; ++i)
-        {
-            float acc = 0.f;
-            for (int o = 0; o < nOut; ++o) acc = fmaf(W[o * 64 + i], dn[o], acc);
-            cur[i] = h[64 * l + i] > 0.f ? acc : 0.f;
-        }
-        for (int i = 0; i < 64; ++i)
-        {
-            nextDelta[i] = cur[i];
-            d[64 * l + i] = cur[i];
-        }
-        dn = nextDelta;
-        nOut = 64;
-    }
-    float* hs = s.h + static_cast<size_t>(b) * 256;
-    for (int i = 0; i < 256; ++i) hs[i] = h[i];
-    float* is = s.in + static_cast<size_t>(b) * GUIDE_IN;
-    for (int i = 0; i < GUIDE_IN; ++i) is[i] = in[i];
-}
-
-// explicit samples (gradient checks)
-__global__ void passExplicitKernel(const float* P, int n, const float* in, const float* k, const float* w,
-                                   BatchScratch s)
-{
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= n) return;
-    float l;
-    samplePass(P, in + static_cast<size_t>(b) * GUIDE_IN, k + 3 * static_cast<size_t>(b), w[b], s, b, l);
-    atomicAdd(s.loss, l);
+    return valid && q == 0 ? -w * logq : 0.f;
 }
 
 // position bin of a record (inputs 0..2 are the position scaled to [-1, 1])
@@ -180,67 +259,200 @@ __global__ void binMeanKernel(int nbins, const float* binSum, const unsigned* bi
     if (b < nbins) binMean[b] = binCount[b] ? binSum[b] / static_cast<float>(binCount[b]) : 0.f;
 }
 
-// a random batch of pilot records, weight I / (mean I * B), or I / (mean I of the bin * B)
-__global__ void passRecordsKernel(const float* P, const GuideRecord* rec, unsigned long long nrec, int B, float invMeanI,
-                                  int nb, const float* binMean, unsigned long long seed, unsigned step, BatchScratch s)
+// the samples of a batch: explicit ones (gradient checks), or random pilot records of weight
+// I / (mean I * B), or I / (mean I of the bin * B)
+struct BatchSource
 {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    U4 r = philox4x32_10(U4{step, static_cast<uint32_t>(b), 0x6d6c70u, 0u}, static_cast<uint32_t>(seed),
-                         static_cast<uint32_t>(seed >> 32));
-    unsigned long long j = ((static_cast<unsigned long long>(r.x) << 32) | r.y) % nrec;
-    const GuideRecord& q = rec[j];
-    float w = q.I * invMeanI;
-    if (nb > 0)
-    {
-        float m = binMean[positionBin(q, nb)];
-        w = m > 0.f ? q.I / m : 0.f;
-    }
-    float l;
-    samplePass(P, q.f, q.k, w / static_cast<float>(B), s, b, l);
-    atomicAdd(s.loss, l);
-}
+    const float *in, *k, *w;  // explicit samples: 8, 3 and 1 floats each
+    const GuideRecord* rec;
+    unsigned long long nrec;
+    float invMeanI;
+    int nb;
+    const float* binMean;
+    unsigned long long seed;
+    unsigned step;
 
-// gradient of one parameter: sum over the batch of delta[b][o] * input[b][i] (or delta for a bias)
-__global__ void weightGradKernel(int B, BatchScratch s, float* grad)
-{
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= GUIDE_NPARAMS) return;
-    int l = 0;
-    while (l + 1 < GUIDE_LAYERS && p >= guideParamOffset(l + 1)) ++l;
-    int local = p - guideParamOffset(l);
-    int nin = guideDimIn(l), nout = guideDimOut(l);
-    int dcol = l + 1 < GUIDE_LAYERS ? 64 * l : 256;
-    float acc = 0.f;
-    if (local < nout * nin)
+    SKG_D void load(int b, int n, float* x, float* dir, float& weight) const
     {
-        int o = local / nin, i = local % nin;
-        for (int b = 0; b < B; ++b)
+        if (in)
         {
-            float x = l == 0 ? s.in[static_cast<size_t>(b) * GUIDE_IN + i] : s.h[static_cast<size_t>(b) * 256 + 64 * (l - 1) + i];
-            acc = fmaf(s.delta[static_cast<size_t>(b) * DELTA_W + dcol + o], x, acc);
+            for (int i = 0; i < GUIDE_IN; ++i) x[i] = in[static_cast<size_t>(b) * GUIDE_IN + i];
+            for (int i = 0; i < 3; ++i) dir[i] = k[3 * static_cast<size_t>(b) + i];
+            weight = w[b];
+            return;
+        }
+        U4 r = philox4x32_10(U4{step, static_cast<uint32_t>(b), 0x6d6c70u, 0u}, static_cast<uint32_t>(seed),
+                             static_cast<uint32_t>(seed >> 32));
+        const GuideRecord& q = rec[((static_cast<unsigned long long>(r.x) << 32) | r.y) % nrec];
+        float wq = q.I * invMeanI;
+        if (nb > 0)
+        {
+            float m = binMean[positionBin(q, nb)];
+            wq = m > 0.f ? q.I / m : 0.f;
+        }
+        for (int i = 0; i < GUIDE_IN; ++i) x[i] = q.f[i];
+        for (int i = 0; i < 3; ++i) dir[i] = q.k[i];
+        weight = wq / static_cast<float>(n);
+    }
+};
+
+template<int S>
+__global__ void __launch_bounds__(GB_THREADS, 1) batchKernel(const float* __restrict__ P, int n, BatchSource src,
+                                                             float* __restrict__ partial)
+{
+    extern __shared__ __align__(16) float sm[];
+    float* X = sm + GB_X;
+    float* H = X + S * GB_LD0;          // 4 hidden layers
+    float* D0 = H + 4 * S * GB_LD;      // delta buffers (the raw outputs start in the first)
+    float* D1 = D0 + S * GB_LD;
+    float* K = D1 + S * GB_LD;          // direction and weight of each sample
+    constexpr int GS = GB_THREADS / S;
+    // the network into its padded rows
+    for (int l = 0; l < GUIDE_LAYERS; ++l)
+    {
+        const int nin = guideDimIn(l), nout = guideDimOut(l), ld = l == 0 ? GB_LD0 : GB_LD;
+        const float* W = P + guideParamOffset(l);
+        for (int i = threadIdx.x; i < nout * nin; i += GB_THREADS) sm[gbW(l) + (i / nin) * ld + i % nin] = W[i];
+        for (int i = threadIdx.x; i < nout; i += GB_THREADS) sm[GB_B + 64 * l + i] = W[nout * nin + i];
+    }
+    float4 G[4][4];  // layers 1 - 4
+    float g0[2] = {0.f, 0.f};  // layer 0: outputs o, o + 32 of input i = t % 8
+    float gb[GUIDE_LAYERS];
+    for (int l = 0; l < 4; ++l)
+        for (int r = 0; r < 4; ++r) G[l][r] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int l = 0; l < GUIDE_LAYERS; ++l) gb[l] = 0.f;
+    float loss = 0.f;
+
+    // an even share of the batch per block
+    const int lo = static_cast<int>(static_cast<long long>(n) * blockIdx.x / gridDim.x);
+    const int hi = static_cast<int>(static_cast<long long>(n) * (blockIdx.x + 1) / gridDim.x);
+    for (int b0 = lo; b0 < hi; b0 += S)
+    {
+        __syncthreads();
+        if (threadIdx.x < S)
+        {
+            float x[GUIDE_IN] = {}, dir[3] = {0.f, 0.f, 1.f}, w = 0.f;
+            if (b0 + static_cast<int>(threadIdx.x) < hi) src.load(b0 + threadIdx.x, n, x, dir, w);
+            for (int i = 0; i < GUIDE_IN; ++i) X[threadIdx.x * GB_LD0 + i] = x[i];
+            for (int i = 0; i < 3; ++i) K[4 * threadIdx.x + i] = dir[i];
+            K[4 * threadIdx.x + 3] = w;
+        }
+        __syncthreads();
+        tileForward<S, GUIDE_IN, GB_LD0, 64, true>(sm + gbW(0), sm + GB_B, X, H);
+        __syncthreads();
+        for (int l = 1; l < 4; ++l)
+        {
+            tileForward<S, 64, GB_LD, 64, true>(sm + gbW(l), sm + GB_B + 64 * l, H + (l - 1) * S * GB_LD, H + l * S * GB_LD);
+            __syncthreads();
+        }
+        tileForward<S, 64, GB_LD, GUIDE_OUT, false>(sm + gbW(4), sm + GB_B + 256, H + 3 * S * GB_LD, D0);
+        __syncthreads();
+        {
+            const int s = threadIdx.x / GS;
+            loss += tileHead<S>(D0 + s * GB_LD, K + 4 * s, K[4 * s + 3], b0 + s < hi, D1 + s * GB_LD);
+        }
+        __syncthreads();
+        // back through the layers: delta_l = (W_{l+1}^T delta_{l+1}) * relu'(h_l)
+        if (threadIdx.x >> 4 < GUIDE_OUT / 4) tileWeights<S>(D1, H + 3 * S * GB_LD, G[3]);
+        gb[4] += tileBias<S>(D1, GUIDE_OUT);
+        tileBackward<S, GUIDE_OUT>(sm + gbW(4), D1, H + 3 * S * GB_LD, D0);
+        __syncthreads();
+        float *d = D0, *dn = D1;
+#pragma unroll
+        for (int l = 3; l >= 1; --l)
+        {
+            tileWeights<S>(d, H + (l - 1) * S * GB_LD, G[l - 1]);
+            gb[l] += tileBias<S>(d, 64);
+            tileBackward<S, 64>(sm + gbW(l), d, H + (l - 1) * S * GB_LD, dn);
+            __syncthreads();
+            float* t = d;
+            d = dn;
+            dn = t;
+        }
+        gb[0] += tileBias<S>(d, 64);
+        const int o = threadIdx.x >> 3, i = threadIdx.x & 7;
+        for (int s = 0; s < S; ++s)
+        {
+            const float x = X[s * GB_LD0 + i];
+            g0[0] = fmaf(d[s * GB_LD + o], x, g0[0]);
+            g0[1] = fmaf(d[s * GB_LD + o + 32], x, g0[1]);
         }
     }
-    else
+    // this block's sums, in the layout of the parameters
+    float* out = partial + static_cast<size_t>(blockIdx.x) * GB_PARTIAL;
+    const int i0 = 4 * (threadIdx.x & 15), o0 = 4 * (threadIdx.x >> 4);
+    for (int r = 0; r < 2; ++r) out[((threadIdx.x >> 3) + 32 * r) * GUIDE_IN + (threadIdx.x & 7)] = g0[r];
+#pragma unroll
+    for (int l = 1; l < GUIDE_LAYERS; ++l)
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            if (o0 + r < guideDimOut(l))
+            {
+                float* at = out + guideParamOffset(l) + (o0 + r) * 64 + i0;
+                at[0] = G[l - 1][r].x;
+                at[1] = G[l - 1][r].y;
+                at[2] = G[l - 1][r].z;
+                at[3] = G[l - 1][r].w;
+            }
+    __syncthreads();
+#pragma unroll
+    for (int l = 0; l < GUIDE_LAYERS; ++l) X[l * GB_THREADS + threadIdx.x] = gb[l];
+    X[GUIDE_LAYERS * GB_THREADS + threadIdx.x] = loss;
+    __syncthreads();
+    for (int t = threadIdx.x; t < 64 * GUIDE_LAYERS; t += GB_THREADS)
     {
-        int o = local - nout * nin;
-        for (int b = 0; b < B; ++b) acc += s.delta[static_cast<size_t>(b) * DELTA_W + dcol + o];
+        const int l = t / 64, oo = t % 64;
+        const float* q = X + l * GB_THREADS + oo;
+        if (oo < guideDimOut(l))
+            out[guideParamOffset(l) + guideDimOut(l) * guideDimIn(l) + oo] = (q[0] + q[64]) + (q[128] + q[192]);
     }
-    grad[p] = acc;
+    if (threadIdx.x < 32)
+    {
+        float v = 0.f;
+        for (int t = threadIdx.x; t < GB_THREADS; t += 32) v += X[GUIDE_LAYERS * GB_THREADS + t];
+        for (int m = 16; m > 0; m >>= 1) v += __shfl_down_sync(0xffffffffu, v, m);
+        if (threadIdx.x == 0) out[GUIDE_NPARAMS] = v;
+    }
 }
 
-__global__ void adamKernel(float* P, const float* g, float* m, float* v, float lr, float b1, float b2, float eps,
-                           float c1, float c2, float clip)
+// grad[p] = the blocks' sums added in block order (p = GUIDE_NPARAMS: the loss), and with `lr` > 0 the
+// Adam step of parameter p
+__global__ void __launch_bounds__(128) gradSumKernel(const float* __restrict__ partial, int blocks, float* grad, float* P,
+                                                     float* m, float* v, float lr, float b1, float b2, float eps, float c1,
+                                                     float c2, float clip)
 {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= GUIDE_NPARAMS) return;
-    float gp = fminf(clip, fmaxf(-clip, g[p]));
+    if (p >= GB_PARTIAL) return;
+    float acc = 0.f;
+#pragma unroll 8
+    for (int b = 0; b < blocks; ++b) acc += partial[static_cast<size_t>(b) * GB_PARTIAL + p];
+    grad[p] = acc;
+    if (!(lr > 0.f) || p >= GUIDE_NPARAMS) return;
+    float gp = fminf(clip, fmaxf(-clip, acc));
     if (!isfinite(gp)) gp = 0.f;
     float mp = b1 * m[p] + (1.f - b1) * gp;
     float vp = b2 * v[p] + (1.f - b2) * gp * gp;
     m[p] = mp;
     v[p] = vp;
     P[p] -= lr * (mp / c1) / (sqrtf(vp / c2) + eps);
+}
+
+// Tiles of 64 samples, which read shared memory half as often per multiply-add, or of 32 for a batch of
+// at most 64 per SM: a block then has one tile of either size, and the small one is done sooner.
+cudaError_t launchBatch(const float* P, int n, const BatchSource& src, float* partial, int numSMs, int* blocks)
+{
+    const bool small = n <= 64 * numSMs;
+    const int S = small ? 32 : 64;
+    const size_t bytes = gbFloats(S) * sizeof(float);
+    const void* f = small ? reinterpret_cast<const void*>(batchKernel<32>) : reinterpret_cast<const void*>(batchKernel<64>);
+    cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    if (e != cudaSuccess) return e;
+    *blocks = std::max(1, std::min(numSMs, (n + S - 1) / S));
+    if (small)
+        batchKernel<32><<<*blocks, GB_THREADS, bytes>>>(P, n, src, partial);
+    else
+        batchKernel<64><<<*blocks, GB_THREADS, bytes>>>(P, n, src, partial);
+    return cudaGetLastError();
 }
 
 // tensor-core forward pass of n explicit samples (tests): 128 samples per CTA
@@ -297,8 +509,7 @@ cudaError_t allocN(T** p, size_t n)
 // ---------------------------------------------------------------------------------------------
 GuideState::~GuideState()
 {
-    void* ps[] = {params, blob, adamM, adamV, grad, records, recCount, scratchIn, scratchH, scratchDelta, lossAcc,
-                  importance, errFlag, binMean};
+    void* ps[] = {params, blob, adamM, adamV, grad, records, recCount, batchIn, partial, importance, errFlag, binMean};
     for (void* p : ps)
         if (p) cudaFree(p);
 }
@@ -311,9 +522,9 @@ cudaError_t guideEnsure(skgpu_ctx* ctx)
     if (e == cudaSuccess) e = allocN(&g->blob, GM_BLOB_BYTES);
     if (e == cudaSuccess) e = allocN(&g->adamM, GUIDE_NPARAMS);
     if (e == cudaSuccess) e = allocN(&g->adamV, GUIDE_NPARAMS);
-    if (e == cudaSuccess) e = allocN(&g->grad, GUIDE_NPARAMS);
+    if (e == cudaSuccess) e = allocN(&g->grad, GB_PARTIAL);
+    if (e == cudaSuccess) e = allocN(&g->partial, static_cast<size_t>(ctx->numSMs) * GB_PARTIAL);
     if (e == cudaSuccess) e = allocN(&g->recCount, 1);
-    if (e == cudaSuccess) e = allocN(&g->lossAcc, 1);
     if (e == cudaSuccess) e = allocN(&g->errFlag, 1);
     if (e == cudaSuccess) e = cudaMemset(g->recCount, 0, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(g->errFlag, 0, sizeof(int));
@@ -362,18 +573,15 @@ cudaError_t guideRepack(skgpu_ctx* ctx)
     return cudaMemcpy(g->blob, blob.data(), blob.size(), cudaMemcpyHostToDevice);
 }
 
-static cudaError_t ensureScratch(GuideState* g, int B)
+// device space for the explicit samples of a batch, kept for the next call (12 floats a sample)
+static cudaError_t ensureBatch(GuideState* g, int n)
 {
-    if (g->scratchRows >= B) return cudaSuccess;
-    cudaFree(g->scratchIn);
-    cudaFree(g->scratchH);
-    cudaFree(g->scratchDelta);
-    g->scratchIn = g->scratchH = g->scratchDelta = nullptr;
-    g->scratchRows = 0;
-    cudaError_t e = allocN(&g->scratchIn, static_cast<size_t>(B) * GUIDE_IN);
-    if (e == cudaSuccess) e = allocN(&g->scratchH, static_cast<size_t>(B) * 256);
-    if (e == cudaSuccess) e = allocN(&g->scratchDelta, static_cast<size_t>(B) * DELTA_W);
-    if (e == cudaSuccess) g->scratchRows = B;
+    if (g->batchRows >= n) return cudaSuccess;
+    cudaFree(g->batchIn);
+    g->batchIn = nullptr;
+    g->batchRows = 0;
+    cudaError_t e = allocN(&g->batchIn, static_cast<size_t>(n) * (GUIDE_IN + 4));
+    if (e == cudaSuccess) g->batchRows = n;
     return e;
 }
 
@@ -381,29 +589,31 @@ cudaError_t guideLossGrad(skgpu_ctx* ctx, int n, const float* in, const float* k
                           float* grad)
 {
     GuideState* g = ctx->guide;
-    cudaError_t e = ensureScratch(g, n);
+    cudaError_t e = ensureBatch(g, n);
     if (e != cudaSuccess) return e;
-    float *dIn = nullptr, *dK = nullptr, *dW = nullptr;
-    e = allocN(&dIn, static_cast<size_t>(n) * GUIDE_IN);
-    if (e == cudaSuccess) e = allocN(&dK, 3 * static_cast<size_t>(n));
-    if (e == cudaSuccess) e = allocN(&dW, n);
-    if (e == cudaSuccess) e = cudaMemcpy(dIn, in, static_cast<size_t>(n) * GUIDE_IN * sizeof(float), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(dK, k, 3 * static_cast<size_t>(n) * sizeof(float), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(dW, w, static_cast<size_t>(n) * sizeof(float), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(g->lossAcc, 0, sizeof(float));
-    BatchScratch s{g->scratchIn, g->scratchH, g->scratchDelta, g->lossAcc};
+    const size_t rows = static_cast<size_t>(n);
+    float *dIn = g->batchIn, *dK = dIn + rows * GUIDE_IN, *dW = dK + 3 * rows;
+    e = cudaMemcpy(dIn, in, rows * GUIDE_IN * sizeof(float), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(dK, k, 3 * rows * sizeof(float), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(dW, w, rows * sizeof(float), cudaMemcpyHostToDevice);
+    BatchSource src{};
+    src.in = dIn;
+    src.k = dK;
+    src.w = dW;
+    int blocks = 0;
+    if (e == cudaSuccess) e = launchBatch(g->params, n, src, g->partial, ctx->numSMs, &blocks);
     if (e == cudaSuccess)
     {
-        passExplicitKernel<<<(n + 127) / 128, 128>>>(g->params, n, dIn, dK, dW, s);
-        weightGradKernel<<<(GUIDE_NPARAMS + 255) / 256, 256>>>(n, s, g->grad);
+        gradSumKernel<<<(GB_PARTIAL + 127) / 128, 128>>>(g->partial, blocks, g->grad, nullptr, nullptr, nullptr, 0.f, 0.f,
+                                                         0.f, 0.f, 1.f, 1.f, 0.f);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpy(loss, g->lossAcc, sizeof(float), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(grad, g->grad, GUIDE_NPARAMS * sizeof(float), cudaMemcpyDeviceToHost);
-    cudaFree(dIn);
-    cudaFree(dK);
-    cudaFree(dW);
-    return e;
+    float out[GB_PARTIAL];
+    if (e == cudaSuccess) e = cudaMemcpy(out, g->grad, sizeof out, cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return e;
+    std::copy(out, out + GUIDE_NPARAMS, grad);
+    *loss = out[GUIDE_NPARAMS];
+    return cudaSuccess;
 }
 
 cudaError_t guideInfer(skgpu_ctx* ctx, int n, const float* in, float* out, int tensorCores, int* deviceErr)
@@ -481,8 +691,6 @@ cudaError_t guideTrain(skgpu_ctx* ctx, int steps, int batch, float lr, unsigned 
     cudaError_t e = guideRecordCount(ctx, &nrec);
     if (e != cudaSuccess) return e;
     if (nrec == 0) return cudaErrorInvalidValue;
-    e = ensureScratch(g, batch);
-    if (e != cudaSuccess) return e;
     // mean downstream luminosity of the records (weights are I / mean I)
     double* dSum = nullptr;
     e = allocN(&dSum, 1);
@@ -521,23 +729,32 @@ cudaError_t guideTrain(skgpu_ctx* ctx, int steps, int batch, float lr, unsigned 
         cudaFree(binCount);
         if (e != cudaSuccess) return e;
     }
-    BatchScratch s{g->scratchIn, g->scratchH, g->scratchDelta, g->lossAcc};
+    BatchSource src{};
+    src.rec = g->records;
+    src.nrec = nrec;
+    src.invMeanI = invMeanI;
+    src.nb = nb;
+    src.binMean = g->binMean;
+    src.seed = seed;
     const float b1 = 0.9f, b2 = 0.999f;
     float lastLoss = 0.f;
     for (int it = 0; it < steps && e == cudaSuccess; ++it)
     {
-        e = cudaMemset(g->lossAcc, 0, sizeof(float));
-        passRecordsKernel<<<(batch + 127) / 128, 128>>>(g->params, g->records, nrec, batch, invMeanI, nb, g->binMean,
-                                                        seed, static_cast<unsigned>(g->adamStep), s);
-        weightGradKernel<<<(GUIDE_NPARAMS + 255) / 256, 256>>>(batch, s, g->grad);
+        src.step = static_cast<unsigned>(g->adamStep);
+        int blocks = 0;
+        e = launchBatch(g->params, batch, src, g->partial, ctx->numSMs, &blocks);
         g->adamStep++;
         float c1 = 1.f - std::pow(b1, static_cast<float>(g->adamStep));
         float c2 = 1.f - std::pow(b2, static_cast<float>(g->adamStep));
-        adamKernel<<<(GUIDE_NPARAMS + 255) / 256, 256>>>(g->params, g->grad, g->adamM, g->adamV, lr, b1, b2, 1e-8f, c1,
-                                                         c2, 10.f);
-        if (e == cudaSuccess) e = cudaGetLastError();
-        if (e == cudaSuccess && (it + 1 == steps)) e = cudaMemcpy(&lastLoss, g->lossAcc, sizeof(float), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess)
+        {
+            gradSumKernel<<<(GB_PARTIAL + 127) / 128, 128>>>(g->partial, blocks, g->grad, g->params, g->adamM, g->adamV, lr,
+                                                             b1, b2, 1e-8f, c1, c2, 10.f);
+            e = cudaGetLastError();
+        }
     }
+    if (e == cudaSuccess && steps > 0)
+        e = cudaMemcpy(&lastLoss, g->grad + GUIDE_NPARAMS, sizeof(float), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = guideRepack(ctx);
     if (lossOut) *lossOut = lastLoss;
     return e;

@@ -21,8 +21,9 @@ struct GuideState
     unsigned long long* recCount = nullptr;
     unsigned long long recCapacity = 0;
 
-    float *scratchIn = nullptr, *scratchH = nullptr, *scratchDelta = nullptr, *lossAcc = nullptr;
-    int scratchRows = 0;
+    float* batchIn = nullptr;         // explicit samples of a batch (12 floats each)
+    int batchRows = 0;
+    float* partial = nullptr;         // per block of a batch: gradient and loss
 
     float* importance = nullptr;      // per-pixel weights of the target frame
     int importanceLen = 0;
