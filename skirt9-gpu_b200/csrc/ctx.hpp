@@ -69,6 +69,7 @@ struct skgpu_ctx
     Wave wave{};
     int waveP = 0, waveGroups = 0, waveStats = 0;
     std::vector<void*> waveBufs;
+    int statsClear = 0;  // slots whose statistics buffers hold no entry (cleared, and left so by runs that succeeded)
     unsigned long long* doneHost = nullptr;  // pinned progress word
 
     // device timing of the stage kernels (skgpu_set_stage_timing)

@@ -47,11 +47,12 @@ struct GraphCache
 };
 
 // wavefront life cycle, one entry per traversal precision (separate translation units, so that
-// the FP64 one can be compiled without FMA contraction)
+// the FP64 one can be compiled without FMA contraction); clearStats: the statistics buffers of the
+// slots may hold entries
 cudaError_t runWaveFP64(int gridKind, const Wave& w, int numSMs, cudaStream_t s, unsigned long long* doneHost,
-                        long long* passes, long long maxPasses, bool useGraph, StageTimer* timer, GraphCache* cache);
+                        long long* passes, long long maxPasses, bool useGraph, StageTimer* timer, GraphCache* cache, bool clearStats);
 cudaError_t runWaveFP32(int gridKind, const Wave& w, int numSMs, cudaStream_t s, unsigned long long* doneHost,
-                        long long* passes, long long maxPasses, bool useGraph, StageTimer* timer, GraphCache* cache);
+                        long long* passes, long long maxPasses, bool useGraph, StageTimer* timer, GraphCache* cache, bool clearStats);
 
 // moments of the grouped per-history statistics of the spill log (n records)
 cudaError_t groupStats(const Wave& w, const StatSpill* groups, unsigned long long n, int numSMs, cudaStream_t s);

@@ -182,6 +182,7 @@ void freeWave(skgpu_ctx* ctx)
     ctx->waveBufs.clear();
     ctx->wave = Wave{};
     ctx->waveP = ctx->waveGroups = ctx->waveStats = 0;
+    ctx->statsClear = 0;
 }
 
 template<typename T>
@@ -1624,11 +1625,15 @@ static int runAndCollect(skgpu_ctx* ctx, const Wave& w, bool useGraph, bool time
                                         ctx->orderIdx, ctx->numSMs, ctx->stream);
         if (eo != cudaSuccess) return fail(ctx, SKGPU_ERR_CUDA, std::string("run: ordering: ") + cudaGetErrorString(eo));
     }
-    cudaError_t e = prec == SKGPU_PREC_FP64_EXACT
-                        ? runWaveFP64(ctx->g.kind, w, ctx->numSMs, ctx->stream, ctx->doneHost, &passes, MAX_PASSES, useGraph, timer,
-                                      &ctx->graphCache)
-                        : runWaveFP32(ctx->g.kind, w, ctx->numSMs, ctx->stream, ctx->doneHost, &passes, MAX_PASSES, useGraph, timer,
-                                      &ctx->graphCache);
+    // the context's own statistics buffers stay clear from one successful run to the next; the static
+    // ones of a run without allocation are shared by every context
+    const bool own = w.pk.skey == ctx->wave.pk.skey;
+    const int clear = own ? ctx->statsClear : 0;
+    const bool clearStats = clear < w.P;
+    if (own && w.anyStats) ctx->statsClear = 0;
+    auto* runWave = prec == SKGPU_PREC_FP64_EXACT ? runWaveFP64 : runWaveFP32;
+    cudaError_t e = runWave(ctx->g.kind, w, ctx->numSMs, ctx->stream, ctx->doneHost, &passes, MAX_PASSES, useGraph, timer,
+                            &ctx->graphCache, clearStats);
     if (e == cudaErrorNotSupported) return fail(ctx, SKGPU_ERR_UNSUPPORTED, "run: no FP32 walker for this grid kind");
     if (e == cudaErrorLaunchTimeout) return fail(ctx, SKGPU_ERR_TIMEOUT, "run: pass limit reached before all histories finished");
     if (e != cudaSuccess) return fail(ctx, SKGPU_ERR_CUDA, std::string("run: ") + cudaGetErrorString(e));
@@ -1665,6 +1670,7 @@ static int runAndCollect(skgpu_ctx* ctx, const Wave& w, bool useGraph, bool time
     if (errFlag & 16) return fail(ctx, SKGPU_ERR_TIMEOUT, "run: a tensor-core wait of the guided-scattering stage gave up");
     if (errFlag & 32) return fail(ctx, SKGPU_ERR_DEVICE, "run: non-finite guided-scattering weight");
     if (errFlag) return fail(ctx, SKGPU_ERR_DEVICE, "run: interaction point outside the grid (device check)");
+    if (own && w.anyStats) ctx->statsClear = std::max(clear, w.P);
     return SKGPU_OK;
 }
 

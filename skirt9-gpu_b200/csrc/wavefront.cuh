@@ -66,14 +66,30 @@ SKG_D void storeRng(const Wave& w, int slot, const Rng& r)
     w.pk.rec[slot].rngSpare = r.spare;
 }
 
-SKG_D void addMoments(double* base, size_t plane, size_t idx, double wsum)
+// w^0 .. w^4 of a history's contribution. An SED has few bins, so that most histories of a run meet in
+// the same five addresses: the warp's lanes that add to one bin are summed first (in a shell of 1e6
+// histories with one bin their atomics took 8 of 20 ms; with this the run takes 14). A frame's lanes
+// rarely meet.
+SKG_D void addMoments(double* base, size_t plane, size_t idx, double wsum, bool shared)
 {
-    double wn = 1.;
-    for (int k = 0; k <= 4; ++k)
+    double sum[5] = {1., wsum, wsum * wsum, wsum * wsum * wsum, wsum * wsum * wsum * wsum};
+    bool lead = true;
+    if (shared)
     {
-        atomicAdd(base + k * plane + idx, wn);
-        wn *= wsum;
+        const unsigned active = __activemask();
+        const unsigned peers = __match_any_sync(active, reinterpret_cast<unsigned long long>(base + idx));
+        lead = (threadIdx.x & 31) == __ffs(peers) - 1;
+        double mine[5];
+        for (int k = 0; k <= 4; ++k)
+        {
+            mine[k] = sum[k];
+            sum[k] = 0.;
+        }
+        for (unsigned rem = peers; rem; rem &= rem - 1)
+            for (int k = 0; k <= 4; ++k) sum[k] += __shfl_sync(peers, mine[k], __ffs(rem) - 1);
     }
+    if (lead)
+        for (int k = 0; k <= 4; ++k) atomicAdd(base + k * plane + idx, sum[k]);
 }
 
 SKG_D void statMoments(const Scene& sc, unsigned long long key, double wsum)
@@ -83,11 +99,11 @@ SKG_D void statMoments(const Scene& sc, unsigned long long key, double wsum)
     int l = static_cast<int>(key & 0xFFFFFF) - 1;
     const InstrDev& in = sc.instr[i];
     if (l < 0)
-        addMoments(in.sedStats, in.nbins, ell, wsum);
+        addMoments(in.sedStats, in.nbins, ell, wsum, true);
     else
     {
         size_t npix = static_cast<size_t>(in.npx) * in.npy;
-        addMoments(in.ifuStats, npix * in.nbins, static_cast<size_t>(l) + static_cast<size_t>(ell) * npix, wsum);
+        addMoments(in.ifuStats, npix * in.nbins, static_cast<size_t>(l) + static_cast<size_t>(ell) * npix, wsum, false);
     }
 }
 
@@ -1065,17 +1081,19 @@ __global__ void __launch_bounds__(256) stepKernel(const __grid_constant__ Wave w
 
 static __global__ void closePassKernel(const __grid_constant__ Wave w, int cur) { closePass(w, cur); }
 
-static __global__ void initPoolKernel(const __grid_constant__ Wave w)
+static __global__ void initPoolKernel(const __grid_constant__ Wave w, int clearStats)
 {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < w.P; t += gridDim.x * blockDim.x)
     {
         w.pk.freeSlots[w.pipelined ? static_cast<size_t>(w.P) + t : t] = t;
-        if (w.anyStats)
-        {
-            w.pk.nstat[t] = 0;
-            for (int a = 0; a < w.statCap; ++a) w.pk.skey[static_cast<size_t>(t) * w.statCap + a] = ~0ULL;
-        }
+        if (clearStats) w.pk.nstat[t] = 0;
     }
+    // the statistics keys: every history leaves its slot's empty, so only new buffers, and those of a run
+    // that failed, need it (1 KB per slot, as much as a run of a few hundred crossings per history moves)
+    if (clearStats)
+        for (size_t t = blockIdx.x * blockDim.x + threadIdx.x; t < static_cast<size_t>(w.P) * w.statCap;
+             t += static_cast<size_t>(gridDim.x) * blockDim.x)
+            w.pk.skey[t] = ~0ULL;
     if (blockIdx.x == 0 && threadIdx.x == 0)
     {
         Control* c = w.ctl;

@@ -180,7 +180,7 @@ std::vector<unsigned char> graphKey(const Wave& w, const WaveLaunch& L, const St
 
 template<class Walker>
 cudaError_t runWave(const Wave& wave, int numSMs, cudaStream_t s, unsigned long long* doneHost, long long* passes,
-                    long long maxPasses, bool useGraph, StageTimer* timer, GraphCache* cache = nullptr)
+                    long long maxPasses, bool useGraph, StageTimer* timer, GraphCache* cache, bool clearStats)
 {
     Wave w = wave;
     WaveLaunch L{};
@@ -217,7 +217,7 @@ cudaError_t runWave(const Wave& wave, int numSMs, cudaStream_t s, unsigned long 
         if (ea != cudaSuccess) return ea;
     }
     if (cache) cache->kernelsPerPass = (L.pipelined ? (L.forced ? 6 : 4) + (L.guided ? 1 : 0) : 7) + (L.guided ? 1 : 0);
-    initPoolKernel<<<L.shadeBlocks, L.threads, 0, s>>>(w);
+    initPoolKernel<<<L.shadeBlocks, L.threads, 0, s>>>(w, w.anyStats && clearStats ? 1 : 0);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (w.count == 0) return cudaStreamSynchronize(s);

@@ -9,22 +9,22 @@ namespace skg {
 
 cudaError_t runWaveFP32(int gridKind, const Wave& w, int numSMs, cudaStream_t s, unsigned long long* doneHost,
                         long long* passes, long long maxPasses, bool useGraph,
-                        StageTimer* timer, GraphCache* cache)
+                        StageTimer* timer, GraphCache* cache, bool clearStats)
 {
     switch (gridKind)
     {
-        case 0: return runWave<CartesianT<float>>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
+        case 0: return runWave<CartesianT<float>>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
         case 1:
-            return w.sc.g.tWallN ? runWave<OctreeT<float>>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache)
-                                 : runWave<OctreeNodeFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 2: return runWave<VoronoiRec32>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 3: return runWave<TetraPlane32>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 4: return runWave<Sphere1DFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 5: return runWave<Cylinder2DFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 6: return runWave<Sphere2DFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 7: return runWave<Sphere3DFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 8: return runWave<Cylinder3DFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 9: return runWave<AdaptiveMeshFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
+            return w.sc.g.tWallN ? runWave<OctreeT<float>>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats)
+                                 : runWave<OctreeNodeFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 2: return runWave<VoronoiRec32>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 3: return runWave<TetraPlane32>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 4: return runWave<Sphere1DFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 5: return runWave<Cylinder2DFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 6: return runWave<Sphere2DFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 7: return runWave<Sphere3DFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 8: return runWave<Cylinder3DFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 9: return runWave<AdaptiveMeshFast>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
     }
     return cudaErrorNotSupported;
 }

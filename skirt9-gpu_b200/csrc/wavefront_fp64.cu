@@ -9,22 +9,22 @@ namespace skg {
 
 cudaError_t runWaveFP64(int gridKind, const Wave& w, int numSMs, cudaStream_t s, unsigned long long* doneHost,
                         long long* passes, long long maxPasses, bool useGraph,
-                        StageTimer* timer, GraphCache* cache)
+                        StageTimer* timer, GraphCache* cache, bool clearStats)
 {
     switch (gridKind)
     {
-        case 0: return runWave<CartesianT<double>>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
+        case 0: return runWave<CartesianT<double>>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
         case 1:
-            return w.sc.g.tWallN ? runWave<OctreeT<double>>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache)
-                                 : runWave<OctreeExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 2: return runWave<VoronoiExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 3: return runWave<TetraExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 4: return runWave<Sphere1DExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 5: return runWave<Cylinder2DExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 6: return runWave<Sphere2DExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 7: return runWave<Sphere3DExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 8: return runWave<Cylinder3DExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
-        case 9: return runWave<AdaptiveMeshExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache);
+            return w.sc.g.tWallN ? runWave<OctreeT<double>>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats)
+                                 : runWave<OctreeExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 2: return runWave<VoronoiExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 3: return runWave<TetraExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 4: return runWave<Sphere1DExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 5: return runWave<Cylinder2DExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 6: return runWave<Sphere2DExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 7: return runWave<Sphere3DExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 8: return runWave<Cylinder3DExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
+        case 9: return runWave<AdaptiveMeshExact>(w, numSMs, s, doneHost, passes, maxPasses, useGraph, timer, cache, clearStats);
     }
     return cudaErrorInvalidValue;
 }
