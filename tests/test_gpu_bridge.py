@@ -198,6 +198,7 @@ def dust_scene(grid, n):
     return ski.dust_curvilinear(n, grid)
 
 
+@needs_build
 @pytest.mark.parametrize("grid", ["voronoi", "tetra", "sphere1d", "sphere2d", "sphere3d", "cylinder2d", "cylinder3d"])
 def test_bridge_dust_emission_other_grids(tmp_path, grid):
     """DustEmission on the Voronoi, tetrahedral, spherical and cylindrical grids through skirt_gpu -g."""
