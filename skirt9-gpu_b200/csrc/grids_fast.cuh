@@ -115,9 +115,9 @@ struct CartesianT : BoxWalker
 
     SKG_D bool next(const GridDev& g)
     {
-        if (state == GS_OUTSIDE) return false;
-        if (state == GS_UNKNOWN)
+        if (state != GS_INSIDE)
         {
+            if (state == GS_OUTSIDE) return false;
             if (!moveInside(g.ext, g.eps)) return false;
             int i = locateClip(g.xb, g.nx + 1, rx);
             int j = locateClip(g.yb, g.ny + 1, ry);
@@ -267,9 +267,9 @@ struct OctreeT : BoxWalker
 
     SKG_D bool next(const GridDev& g)
     {
-        if (state == GS_OUTSIDE) return false;
-        if (state == GS_UNKNOWN)
+        if (state != GS_INSIDE)
         {
+            if (state == GS_OUTSIDE) return false;
             if (!moveInside(g.ext, g.eps)) return false;
             if (!(cell >= 0 && ds == 0. && holds(g, cell)))
             {
@@ -490,9 +490,9 @@ struct VoronoiRec32 : GenBase
 
     SKG_D bool next(const GridDev& g)
     {
-        if (state == GS_OUTSIDE) return false;
-        if (state == GS_UNKNOWN)
+        if (state != GS_INSIDE)
         {
+            if (state == GS_OUTSIDE) return false;
             if (!moveInside(g.ext, g.eps)) return false;
             if (!locateRec(g, (hint >= 0 && ds == 0.) ? hint : -1))
             {
@@ -752,9 +752,9 @@ struct TetraPlane32 : GenBase
 
     SKG_D bool next(const GridDev& g)
     {
-        if (state == GS_OUTSIDE) return false;
-        if (state == GS_UNKNOWN)
+        if (state != GS_INSIDE)
         {
+            if (state == GS_OUTSIDE) return false;
             if (!moveInside(g.ext, g.eps)) return false;
             mr = (hint >= 0 && ds == 0.) ? hint : tetraLocate(g, rx, ry, rz);
             ef = -1;

@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __g
     Acc tau = 0, fA = 0, fB = 0, fC = 0, sext = 0;
     int iA = -1, nseg = 0;
     unsigned cross = 0, rfStores = 0;  // flushed to the counters before they can overflow
-    int guard = 0;
+    int guard = 0;  // crossings of the present ray
 
     while (true)
     {
@@ -427,10 +427,11 @@ __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __g
         if (kind < 0) continue;
 
         bool got = wk.next(scn().g);
-        bool done = !got;
+        // a ray that has left the grid has no further segment
+        bool done = !got || wk.state == GS_OUTSIDE;
         if (got)
         {
-            cross++;
+            ++guard;
             int m = wk.m;
             Acc ds = static_cast<Acc>(wk.ds);
             if (isPeel())
@@ -492,11 +493,12 @@ __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __g
                         b.s[idx] = static_cast<double>(s0 + ((fA - tau0) / (tau - tau0)) * (fB - s0));
                         b.found[idx] = 1;
                         kind = -1;
+                        cross += guard;
                         continue;
                     }
                 }
             }
-            if (++guard > (1 << 20))
+            if (guard > (1 << 20))
             {
                 // a traversal that does not end: report the first few (task kind, start point and
                 // direction, last cell) and stop it; the run returns SKGPU_ERR_TIMEOUT
@@ -529,6 +531,7 @@ __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __g
                 b.found[idx] = 0;
             }
             kind = -1;
+            cross += guard;
             if ((cross | rfStores) & 0x80000000u)
             {
                 atomicAdd(&w.ctl->counters[1], static_cast<unsigned long long>(cross));
