@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/skgpu.h"
+#include "host_pool.hpp"
 #include "internal.hpp"
 #include "stage_timer.hpp"
 
@@ -37,6 +38,7 @@ struct skgpu_ctx
 
     double *mixLb = nullptr, *mixExt = nullptr, *mixSca = nullptr, *mixG = nullptr;
     int nmix = 0;
+    std::vector<double> mixLbHost, mixExtHost;
 
     int nrf = 0, rfNb = 0;
     double* rfB = nullptr;
@@ -46,7 +48,9 @@ struct skgpu_ctx
 
     std::vector<SourceDev> srcHost;
     SourceDev* src = nullptr;
-    double *tabL = nullptr, *tabA = nullptr, *tabB = nullptr, *radR = nullptr, *radP = nullptr;
+    double *tabL = nullptr, *tabA = nullptr, *tabB = nullptr, *radR = nullptr, *radP = nullptr;  // within srcBuf
+    unsigned char* srcBuf = nullptr;  // the source records and their tables
+    size_t srcBytes = 0;
 
     std::vector<InstrDev> instrHost;
     InstrDev* instr = nullptr;
@@ -76,9 +80,13 @@ struct skgpu_ctx
     StageTimer timer;
     bool timerEvents = false;
 
-    // pinned staging of the tally read-back: the copy of one chunk overlaps the host add of the previous
+    // pinned staging of the large host arrays: the copy of one chunk overlaps the host's work on another
     double* pin[2] = {nullptr, nullptr};
     cudaEvent_t pinEv[2] = {nullptr, nullptr};
+    skg::HostPool pool;
+    // rays of skgpu_trace_paths / skgpu_optical_depths: two chunks, on the device and pinned
+    unsigned char *rayDev[2] = {nullptr, nullptr}, *rayPin[2] = {nullptr, nullptr};
+    size_t rayBytes = 0;
 
     // launch shape set by skgpu_set_launch_shape (0: defaults)
     int shapePool = 0, shapeTraceBlocks = 0, shapeShadeBlocks = 0, shapeRefill = 0;
