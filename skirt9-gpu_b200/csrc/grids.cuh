@@ -821,24 +821,16 @@ struct Sphere1DExact : GenBase
                 if (i > imin) inwards = true;
             }
         }
-        if (inwards)
-        {
-            double rN = rv[i];
-            double qN = -sqrt(xmul(xsub(rN, p), xadd(rN, p)));
-            m = i;
-            ds = xsub(qN, q);
-            i--;
-            q = qN;
-            if (i <= imin) inwards = false;
-            return true;
-        }
-        double rN = rv[i + 1];
-        double qN = sqrt(xmul(xsub(rN, p), xadd(rN, p)));
+        // inwards to the next smaller shell, else outwards to the next larger one
+        const double rN = inwards ? rv[i] : rv[i + 1];
+        const double w = sqrt(xmul(xsub(rN, p), xadd(rN, p)));
+        const double qN = inwards ? -w : w;
         m = i;
         ds = xsub(qN, q);
-        i++;
         q = qN;
-        if (i >= nr) state = GS_OUTSIDE;
+        i += inwards ? -1 : 1;
+        if (!inwards && i >= nr) state = GS_OUTSIDE;
+        if (inwards && i <= imin) inwards = false;
         return true;
     }
 };
@@ -855,8 +847,22 @@ struct Cylinder2DExact : GenBase
     static constexpr int kMinBlocks = 4;
     static constexpr int kRefillMin = 16;  // waiting lanes before a warp takes new tasks
     double cR, cz, kq, kzc, p, q;
+    double ikq, ikz;  // reciprocals of kq and kzc (0: to be divided by)
+    double qN, zN;    // the next cylinder and plane on the ray: only the one just crossed is computed anew
     int i, k, imin;
     bool up, in;
+
+    // a / b by the reciprocal ib, the correctly rounded quotient; |b| < 1e-100, whose quotients may leave
+    // the range in which qdiv is exact, has none
+    SKG_D static double ratio(double a, double b, double ib) { return ib != 0. ? qdiv(a, b, ib) : a / b; }
+    SKG_D static double recip(double b) { return fabs(b) > 1e-100 ? 1.0 / b : 0.; }
+
+    SKG_D void radial(const GridDev& g)
+    {
+        double RN = in ? g.cRv[i] : g.cRv[i + 1];
+        double w = sqrt(xmul(xsub(RN, p), xadd(RN, p)));
+        qN = in ? -w : w;
+    }
 
     SKG_D void start(const GridDev&, double x, double y, double z, double ux, double uy, double uz, int = -1)
     {
@@ -937,41 +943,32 @@ struct Cylinder2DExact : GenBase
                 imin = locateNR(Rv, NR + 1, p);
                 if (i > imin) in = true;
             }
+            ikq = recip(kq);
+            ikz = recip(kzc);
+            radial(g);
+            zN = up ? zv[k + 1] : zv[k];
             if (ds > 0.) return true;
         }
-        double RN = in ? Rv[i] : Rv[i + 1];
-        double w = sqrt(xmul(xsub(RN, p), xadd(RN, p)));
-        double qN = in ? -w : w;
-        double zN = up ? zv[k + 1] : zv[k];
         int mc = i < 0 ? -1 : k + Nz * i;  // Cylinder2DSpatialGrid::index
-        double dsq = xsub(qN, q) / kq;
-        double dsz = xsub(zN, cz) / kzc;
+        double dsq = ratio(xsub(qN, q), kq, ikq);
+        double dsz = ratio(xsub(zN, cz), kzc, ikz);
+        m = mc;
         if (dsq < dsz)
         {
-            m = mc;
             ds = dsq;
-            if (in)
+            i += in ? -1 : 1;
+            if (!in && i >= NR)
+                state = GS_OUTSIDE;
+            else
             {
-                i--;
                 q = qN;
                 cz = xadd(cz, xmul(kzc, dsq));
                 if (i <= imin) in = false;
-            }
-            else
-            {
-                i++;
-                if (i >= NR)
-                    state = GS_OUTSIDE;
-                else
-                {
-                    q = qN;
-                    cz = xadd(cz, xmul(kzc, dsq));
-                }
+                radial(g);
             }
         }
         else
         {
-            m = mc;
             ds = dsz;
             k += up ? 1 : -1;
             if (up ? k >= Nz : k < 0)
@@ -980,6 +977,7 @@ struct Cylinder2DExact : GenBase
             {
                 q = xadd(q, xmul(kq, dsz));
                 cz = zN;
+                zN = up ? zv[k + 1] : zv[k];
             }
         }
         return true;
