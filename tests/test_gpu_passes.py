@@ -1,0 +1,148 @@
+"""GPU tests of the pipelined passes and of the buffers that a context keeps between calls.
+
+- The pipelined passes (untimed runs) give the tallies of the plain passes (runs with stage timing):
+  every history draws from its own stream, so both trace the same histories and the tallies differ only
+  by the order of their FP64 additions (1e-12 of the largest entry; a bin sums at most 1e4 terms of
+  one sign, whose rounding errors stay below 1e4 x 1.1e-16).
+- Statistics buffers that a run left behind serve a later run with more slots.
+- Rays in any number, around the chunks of the path entry points, give what one ray at a time gives.
+- A radiation field comes back as it was uploaded, and one with a non-finite value changes nothing.
+"""
+import numpy as np
+import pytest
+
+from skgpu import Scene, SkgpuError, abi, batch
+
+pytestmark = pytest.mark.gpu
+
+
+def tallies(res):
+    out = []
+    for ins in res.instruments:
+        out += [ins["total"].ravel()] + ([ins["stats"].ravel()] if ins["stats"] is not None else [])
+    return out + ([res.rf.ravel()] if res.rf is not None else [])
+
+
+def assert_same(a, b):
+    for x, y in zip(tallies(a), tallies(b)):
+        assert np.allclose(x, y, rtol=1e-12, atol=1e-12 * np.abs(y).max())
+
+
+def timed(be, run):
+    abi.set_stage_timing(be, 2)
+    try:
+        return run()
+    finally:
+        abi.set_stage_timing(be, 0)
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64_EXACT, abi.PREC_FP32])
+@pytest.mark.parametrize("name,stats,forced,explicit", [("shell_c16.npz", 1, True, False), ("shell_c16.npz", 0, True, True),
+                                                        ("shell_c16.npz", 0, False, False), ("stats_octree.npz", 1, True, False),
+                                                        ("stats_voronoi.npz", 0, True, False),
+                                                        ("paths_cylinder2d.npz", 1, False, True)])
+@pytest.mark.parametrize("n", [1, 333, 20000])
+def test_pipelined_equals_plain_passes(golden, gpu_backend, name, stats, forced, explicit, precision, n):
+    sc = Scene.from_export(golden(name))
+    sc.force_scattering, sc.explicit_absorption = forced, explicit
+    for ins in sc.instruments:
+        ins["stats"] = stats
+    sc.upload(gpu_backend)
+    a = sc.run(gpu_backend, n, seed=5, precision=precision)
+    b = timed(gpu_backend, lambda: sc.run(gpu_backend, n, seed=5, precision=precision))
+    assert a.counters["crossings"] == b.counters["crossings"]
+    assert a.counters["scatterings"] == b.counters["scatterings"]
+    assert a.counters["peel_detections"] == b.counters["peel_detections"]
+    assert_same(a, b)
+
+
+@pytest.mark.parametrize("slots", [256, 1000])
+def test_pipelined_passes_refill_a_small_pool(golden, gpu_backend, slots):
+    """More histories than slots: every slot is freed and launched into again many times."""
+    sc = Scene.from_export(golden("shell_c16.npz"))
+    sc.upload(gpu_backend)
+    a = sc.run(gpu_backend, 30001, seed=2, precision=abi.PREC_FP32)
+    abi.set_launch_shape(gpu_backend, slots)
+    b = sc.run(gpu_backend, 30001, seed=2, precision=abi.PREC_FP32)
+    assert b.counters["histories"] == 30001
+    assert_same(a, b)
+
+
+def test_pipelined_batch_equals_plain_passes(golden):
+    scenes = [Scene.from_export(golden("shell_c16.npz")) for _ in range(2)]
+    scenes[1].force_scattering = False
+    bes = [abi.Backend() for _ in scenes]
+    for sc, be in zip(scenes, bes):
+        sc.upload(be)
+    run = lambda: batch.run_batch(scenes, bes, [5000, 777], [3, 4])
+    for a, b in zip(run(), timed(bes[0], run)):
+        assert_same(a, b)
+
+
+def test_statistics_buffers_of_growing_runs(golden, gpu_backend, oracle_backend):
+    """Slots that an earlier, smaller run never used start with empty statistics keys."""
+    sc = Scene.from_export(golden("shell_c16.npz"))
+    for be in (gpu_backend, oracle_backend):
+        sc.upload(be)
+    for n in (3000, 500, 3000, 4000):
+        a, b = sc.run(gpu_backend, n, seed=n), sc.run(oracle_backend, n, seed=n)
+        for x, y in zip(a.instruments, b.instruments):
+            assert np.array_equal(x["stats"][0], y["stats"][0])
+
+
+@pytest.mark.parametrize("n", [1, 2, 299592, 299593, 299594, 600001])
+def test_optical_depths_in_chunks(golden, gpu_backend, n):
+    """16 MB hold 299 593 rays of 56 bytes."""
+    z = golden("paths_cartesian_c16.npz")
+    sc = Scene.from_export(z)
+    sc.upload(gpu_backend)
+    rays = z["rays"]
+    few = gpu_backend.optical_depths(rays, 0.55e-6)
+    at = np.arange(n) % len(rays)
+    assert np.array_equal(gpu_backend.optical_depths(rays[at], 0.55e-6), few[at])
+
+
+@pytest.mark.parametrize("n,segments", [(1, 64), (400, 64), (21000, 64), (3, 700000)])
+def test_path_segments_in_chunks(golden, gpu_backend, n, segments):
+    """16 MB hold 20 460 rays of 64 segments, and one of 700 000."""
+    z = golden("paths_cartesian_c16.npz")
+    Scene.from_export(z).upload(gpu_backend)
+    rays = z["rays"]
+    count, m, ds = gpu_backend.trace_paths(rays, 64)
+    at = np.arange(n) % len(rays)
+    c, mm, dd = gpu_backend.trace_paths(rays[at], segments)
+    assert np.array_equal(c, count[at])
+    w = min(64, segments)
+    assert np.array_equal(mm[:, :w], m[at]) and np.array_equal(dd[:, :w], ds[at])
+    assert not mm[:, w:].any() and not dd[:, w:].any()
+
+
+@pytest.mark.parametrize("bins", [1, 31, 32, 33, 70])
+def test_radiation_field_round_trip(golden, gpu_backend, bins):
+    sc = Scene.from_export(golden("shell_c16.npz"))
+    sc.upload(gpu_backend)
+    borders = np.linspace(1e-7, 1e-5, bins + 1)
+    gpu_backend.upload_rf_grid(bins, borders, np.r_[-1, np.arange(bins), -1].astype(np.int32))
+    rf = np.random.default_rng(bins).uniform(size=(len(sc.density), bins))
+    gpu_backend.upload_radiation_field(rf)
+    assert np.array_equal(gpu_backend.fetch_radiation_field(rf.size).reshape(rf.shape), rf)
+    bad = rf.copy()
+    bad.flat[-1] = np.inf
+    with pytest.raises(SkgpuError):
+        gpu_backend.upload_radiation_field(bad)
+    assert np.array_equal(gpu_backend.fetch_radiation_field(rf.size).reshape(rf.shape), rf)
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 65, 4736, 9472, 9473, 20001])
+def test_guide_gradient_batch_sizes(gpu_backend, n):
+    """Tiles of 32 and 64 samples, whole and ragged, one and several per block (148 SMs: the larger tile
+    from 9 473 samples on). FP32 sums of n terms of about one size: 1e-5 of the largest entry."""
+    import guide_oracle as go
+    from test_gpu_guide import _batch
+    p = go.random_params(4).astype(np.float32)
+    abi.guide_init(gpu_backend, p)
+    x, k, w = _batch(n, n)
+    loss, grad = abi.guide_loss_grad(gpu_backend, x, k, w)
+    lo, gr = go.loss_grad(p.astype(float), x.astype(float), k.astype(float), w.astype(float))
+    assert loss == pytest.approx(lo, rel=1e-5)
+    assert np.abs(grad - gr).max() <= 1e-5 * np.abs(gr).max() + 1e-5 * np.sqrt(np.mean(gr ** 2))
