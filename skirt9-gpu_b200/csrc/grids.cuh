@@ -125,9 +125,8 @@ struct alignas(128) TetRec
 {
     double c[4];
     float n[12];
-    int nb[4];    // neighbour across face f, -1 on the hull
-    int nface;    // neighbour's face index for face f in bits 8f..8f+7
-    int pad[7];
+    int to[4];    // across face f: 4 x neighbour + the face's index on its side, -1 on the hull
+    int pad[8];
 };
 static_assert(sizeof(TetRec) == 128, "one cache line per tetrahedron");
 
@@ -137,6 +136,10 @@ static_assert(sizeof(TetRec) == 128, "one cache line per tetrahedron");
 struct GenBase
 {
     using Acc = double;  // accumulator type of optical depth and path length along the walk
+    // the traversal kernel takes a ray whose state is outside after a segment as ended, without the step
+    // that would say so: 5 % faster for the tetrahedral production walker, no faster for the others, and
+    // 1.6x slower for the FP64 tetrahedral one (its lanes no longer meet after a step)
+    static constexpr bool kEndsOutside = false;
     // the cell of a launched packet is found once, by the launch stage, instead of by each of its rays
     static constexpr bool kLocates = false;
     SKG_D static int locate(const GridDev&, double, double, double) { return -1; }

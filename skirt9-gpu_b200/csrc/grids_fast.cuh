@@ -601,6 +601,15 @@ struct VoronoiRec32 : GenBase
 };
 
 
+// 32 bytes of read-only memory in one load. A gather of records costs the L1 a wavefront per lane and
+// load, whatever the load's size: half as many loads of twice the size.
+SKG_D void load32(const void* p, unsigned (&v)[8])
+{
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+        : "l"(p));
+}
+
 // ---------------------------------------------------------------------------------------------
 // Tetrahedral mesh, production walker (TetraMeshSpatialGrid::MySegmentGenerator::next,
 // TetraMeshSpatialGrid.cpp:688-831). Every step reads one 128-byte record (TetRec) of the current
@@ -621,29 +630,29 @@ struct TetRegs
 {
     double c[4];
     float n[12];
-    int nb[4];
-    int nface;
+    int to[4];
 
     SKG_D static TetRegs load(const TetRec* rec)
     {
-        const float4* q = reinterpret_cast<const float4*>(rec);
-        float4 a = __ldg(q), b = __ldg(q + 1), n0 = __ldg(q + 2), n1 = __ldg(q + 3), n2 = __ldg(q + 4), nb = __ldg(q + 5),
-               nf = __ldg(q + 6);
+        unsigned v[8], u[8], t8[8];
+        load32(rec->c, v);
+        load32(rec->n, u);
+        load32(rec->n + 8, t8);
         TetRegs t;
-        t.c[0] = __hiloint2double(__float_as_int(a.y), __float_as_int(a.x));
-        t.c[1] = __hiloint2double(__float_as_int(a.w), __float_as_int(a.z));
-        t.c[2] = __hiloint2double(__float_as_int(b.y), __float_as_int(b.x));
-        t.c[3] = __hiloint2double(__float_as_int(b.w), __float_as_int(b.z));
-        t.n[0] = n0.x; t.n[1] = n0.y; t.n[2] = n0.z; t.n[3] = n0.w;
-        t.n[4] = n1.x; t.n[5] = n1.y; t.n[6] = n1.z; t.n[7] = n1.w;
-        t.n[8] = n2.x; t.n[9] = n2.y; t.n[10] = n2.z; t.n[11] = n2.w;
-        t.nb[0] = __float_as_int(nb.x); t.nb[1] = __float_as_int(nb.y);
-        t.nb[2] = __float_as_int(nb.z); t.nb[3] = __float_as_int(nb.w);
-        t.nface = __float_as_int(nf.x);
+#pragma unroll
+        for (int f = 0; f < 4; ++f)
+        {
+            t.c[f] = __hiloint2double(v[2 * f + 1], v[2 * f]);
+            t.n[8 + f] = __uint_as_float(t8[f]);
+            t.to[f] = static_cast<int>(t8[4 + f]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t.n[i] = __uint_as_float(u[i]);
         return t;
     }
 
-    SKG_D int neighbour(int f) const { return f == 0 ? nb[0] : f == 1 ? nb[1] : f == 2 ? nb[2] : nb[3]; }
+    // TetRec::to of face f
+    SKG_D int across(int f) const { return f == 0 ? to[0] : f == 1 ? to[1] : f == 2 ? to[2] : to[3]; }
 
     // positive when (x, y, z) lies outside face F's plane
     template<int F>
@@ -672,7 +681,7 @@ SKG_D int tetraLocate(const GridDev& g, double x, double y, double z)
         if ((e = r.excess<2>(x, y, z)) > worst) { worst = e; f = 2; }
         if ((e = r.excess<3>(x, y, z)) > worst) { worst = e; f = 3; }
         if (f < 0) return t;
-        t = r.neighbour(f);
+        t = r.across(f) >> 2;
     }
     return tetraCellIndex(g, x, y, z);  // walk left the hull or did not settle: the reference's block scan
 }
@@ -684,6 +693,7 @@ struct TetraPlane32 : GenBase
 {
     using Acc = float;
     static constexpr int kMinBlocks = SKG_TETRA32_MIN_BLOCKS;
+    static constexpr bool kEndsOutside = true;
     static constexpr int kRefillMin = 8;  // waiting lanes before a warp takes new tasks
     // bound on the displacement of a float plane from its exact one, in units of eps (1e-12 of the
     // domain diagonal): 2^-24 per normal component over at most the diagonal, with margin
@@ -795,18 +805,17 @@ struct TetraPlane32 : GenBase
             // Between two interior faces either choice continues the walk from the same point; only
             // in a tetrahedron on the hull can a float decision end the path where the reference's
             // goes on (or the reverse), so only there is the decision tested, in a second pass.
-            if (lf >= 0 && ((r.nb[0] | r.nb[1] | r.nb[2] | r.nb[3]) >= 0 || !ambiguous(r, rx, ry, rz, tol)))
+            if (lf >= 0 && ((r.to[0] | r.to[1] | r.to[2] | r.to[3]) >= 0 || !ambiguous(r, rx, ry, rz, tol)))
             {
-                int nt = r.neighbour(lf);
-                int nf = (r.nface >> (8 * lf)) & 0xff;
+                const int to = r.across(lf);
                 if (best > 0.f)
                 {
                     m = mr;
                     ds = best;
                     propagater(ds);
                 }
-                mr = nt;
-                ef = nf;
+                mr = to >> 2;
+                ef = to & 3;
                 if (mr < 0)
                 {
                     // the reference drops the final in-mesh segment when the path leaves the hull

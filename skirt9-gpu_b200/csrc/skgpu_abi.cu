@@ -1204,6 +1204,7 @@ int skgpu_upload_grid_tetra(skgpu_ctx* ctx, int32_t num_vertices, const double* 
     if (num_vertices < 4 || num_tetra < 1 || !vertices || !tetra_vertices || !face_normals || !face_ntetra
         || !face_nface || !extent)
         return fail(ctx, SKGPU_ERR_ARG, "tetra: missing arrays");
+    if (num_tetra >= 1 << 29) return fail(ctx, SKGPU_ERR_ARG, "tetra: more than 2^29 - 1 tetrahedra (172 GB on the device)");
     size_t nt = static_cast<size_t>(num_tetra);
     for (size_t q = 0; q < 4 * nt; ++q)
     {
@@ -1264,13 +1265,11 @@ int skgpu_upload_grid_tetra(skgpu_ctx* ctx, int32_t num_vertices, const double* 
     {
         TetRec& r = rec[t];
         std::memset(&r, 0, sizeof r);
-        r.nface = 0;
         for (int f = 0; f < 4; ++f)
         {
             int nb = face_ntetra[4 * t + f];
             int nf = face_nface[4 * t + f];
-            r.nb[f] = nb;
-            r.nface |= (nb >= 0 ? (nf & 0xff) : 0) << (8 * f);
+            r.to[f] = nb >= 0 ? 4 * nb + nf : -1;
             size_t owner = t;
             int of = f;
             double sign = 1.0;

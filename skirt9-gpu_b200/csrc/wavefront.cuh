@@ -427,8 +427,7 @@ __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __g
         if (kind < 0) continue;
 
         bool got = wk.next(scn().g);
-        // a ray that has left the grid has no further segment
-        bool done = !got || wk.state == GS_OUTSIDE;
+        bool done = !got || (Walker::kEndsOutside && wk.state == GS_OUTSIDE);
         if (got)
         {
             ++guard;
