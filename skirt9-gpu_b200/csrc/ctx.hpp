@@ -82,11 +82,12 @@ struct skgpu_ctx
 
     // pinned staging of the large host arrays: the copy of one chunk overlaps the host's work on another
     double* pin[2] = {nullptr, nullptr};
+    size_t pinDoubles = 0;
     cudaEvent_t pinEv[2] = {nullptr, nullptr};
     skg::HostPool pool;
-    // rays of skgpu_trace_paths / skgpu_optical_depths: two chunks, on the device and pinned
-    unsigned char *rayDev[2] = {nullptr, nullptr}, *rayPin[2] = {nullptr, nullptr};
-    size_t rayBytes = 0;
+    // rays and results of skgpu_optical_depths: 7 doubles per row
+    double* rayDev = nullptr;
+    size_t rayRows = 0;
 
     // launch shape set by skgpu_set_launch_shape (0: defaults)
     int shapePool = 0, shapeTraceBlocks = 0, shapeShadeBlocks = 0, shapeRefill = 0;

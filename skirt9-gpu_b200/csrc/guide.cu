@@ -437,9 +437,15 @@ __global__ void __launch_bounds__(128) gradSumKernel(const float* __restrict__ p
     P[p] -= lr * (mp / c1) / (sqrtf(vp / c2) + eps);
 }
 
+template<typename T>
+cudaError_t allocN(T** p, size_t n)
+{
+    return cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(n, 1) * sizeof(T));
+}
+
 // Tiles of 64 samples, which read shared memory half as often per multiply-add, or of 32 for a batch of
 // at most 64 per SM: a block then has one tile of either size, and the small one is done sooner.
-cudaError_t launchBatch(const float* P, int n, const BatchSource& src, float* partial, int numSMs, int* blocks)
+cudaError_t launchBatch(GuideState* g, int n, const BatchSource& src, int numSMs, int* blocks)
 {
     const bool small = n <= 64 * numSMs;
     const int S = small ? 32 : 64;
@@ -448,10 +454,19 @@ cudaError_t launchBatch(const float* P, int n, const BatchSource& src, float* pa
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     if (e != cudaSuccess) return e;
     *blocks = std::max(1, std::min(numSMs, (n + S - 1) / S));
+    if (g->partialBlocks < *blocks)
+    {
+        cudaFree(g->partial);
+        g->partial = nullptr;
+        g->partialBlocks = 0;
+        e = allocN(&g->partial, static_cast<size_t>(*blocks) * GB_PARTIAL);
+        if (e != cudaSuccess) return e;
+        g->partialBlocks = *blocks;
+    }
     if (small)
-        batchKernel<32><<<*blocks, GB_THREADS, bytes>>>(P, n, src, partial);
+        batchKernel<32><<<*blocks, GB_THREADS, bytes>>>(g->params, n, src, g->partial);
     else
-        batchKernel<64><<<*blocks, GB_THREADS, bytes>>>(P, n, src, partial);
+        batchKernel<64><<<*blocks, GB_THREADS, bytes>>>(g->params, n, src, g->partial);
     return cudaGetLastError();
 }
 
@@ -496,12 +511,6 @@ __global__ void sumRecordsKernel(const GuideRecord* rec, unsigned long long n, d
     if ((threadIdx.x & 31) == 0) atomicAdd(sumI, v);
 }
 
-template<typename T>
-cudaError_t allocN(T** p, size_t n)
-{
-    return cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(n, 1) * sizeof(T));
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------------------------
@@ -523,7 +532,6 @@ cudaError_t guideEnsure(skgpu_ctx* ctx)
     if (e == cudaSuccess) e = allocN(&g->adamM, GUIDE_NPARAMS);
     if (e == cudaSuccess) e = allocN(&g->adamV, GUIDE_NPARAMS);
     if (e == cudaSuccess) e = allocN(&g->grad, GB_PARTIAL);
-    if (e == cudaSuccess) e = allocN(&g->partial, static_cast<size_t>(ctx->numSMs) * GB_PARTIAL);
     if (e == cudaSuccess) e = allocN(&g->recCount, 1);
     if (e == cudaSuccess) e = allocN(&g->errFlag, 1);
     if (e == cudaSuccess) e = cudaMemset(g->recCount, 0, sizeof(unsigned long long));
@@ -601,7 +609,7 @@ cudaError_t guideLossGrad(skgpu_ctx* ctx, int n, const float* in, const float* k
     src.k = dK;
     src.w = dW;
     int blocks = 0;
-    if (e == cudaSuccess) e = launchBatch(g->params, n, src, g->partial, ctx->numSMs, &blocks);
+    if (e == cudaSuccess) e = launchBatch(g, n, src, ctx->numSMs, &blocks);
     if (e == cudaSuccess)
     {
         gradSumKernel<<<(GB_PARTIAL + 127) / 128, 128>>>(g->partial, blocks, g->grad, nullptr, nullptr, nullptr, 0.f, 0.f,
@@ -742,7 +750,7 @@ cudaError_t guideTrain(skgpu_ctx* ctx, int steps, int batch, float lr, unsigned 
     {
         src.step = static_cast<unsigned>(g->adamStep);
         int blocks = 0;
-        e = launchBatch(g->params, batch, src, g->partial, ctx->numSMs, &blocks);
+        e = launchBatch(g, batch, src, ctx->numSMs, &blocks);
         g->adamStep++;
         float c1 = 1.f - std::pow(b1, static_cast<float>(g->adamStep));
         float c2 = 1.f - std::pow(b2, static_cast<float>(g->adamStep));

@@ -24,6 +24,7 @@ struct GuideState
     float* batchIn = nullptr;         // explicit samples of a batch (12 floats each)
     int batchRows = 0;
     float* partial = nullptr;         // per block of a batch: gradient and loss
+    int partialBlocks = 0;
 
     float* importance = nullptr;      // per-pixel weights of the target frame
     int importanceLen = 0;

@@ -186,33 +186,83 @@ void freeWave(skgpu_ctx* ctx)
     ctx->statsClear = 0;
 }
 
-// pinned staging buffers: 16 MB each, so that a chunk's copy and the host's work on another overlap also
-// for the arrays of a small segment
-constexpr size_t PIN_DOUBLES = size_t(2) << 20;
-// doubles that a host core takes at least: a copy into pinned memory scales further than an addition
-// into the caller's array, whose pages may have to be mapped first
-constexpr size_t COPY_GRAIN = size_t(1) << 16, ADD_GRAIN = size_t(1) << 18;
+// Pinned staging buffers, two of 4 MB for arrays of up to 32 MB, of 16 MB up to 128 MB, of 32 MB above: a
+// chunk's copy and the host's work on another overlap, and a context pays for pinned memory what its
+// arrays are worth (0.8 ms per MB; two of 64 MB from the first fetch on made a first pass 100 ms longer).
+// Arrays of up to 64 KB go without.
+constexpr size_t PLAIN_DOUBLES = size_t(1) << 13;
 
-int ensurePin(skgpu_ctx* ctx)
+// Doubles that a host core takes at least (0.5 MB).
+constexpr size_t COPY_GRAIN = size_t(1) << 16;
+
+// Maps the pages of a host array for writing, without changing it. An array that nobody wrote to yet (numpy's
+// zeros) has no pages: the load of an addition maps the zero page and its store then faults again and has
+// every core drop the first mapping. 64 MB of it added by 16 cores: 11.1 ms, with the pages written to first
+// 2.9 ms, 1.5 ms with large pages. A core takes 2 MB, a large page, since cores that meet in one that is not
+// mapped each clear one for it; arrays below 4 MB, which numpy leaves to small pages, go by 0.25 MB.
+void mapPages(skgpu_ctx* ctx, double* host, size_t n)
 {
-    for (int i = 0; i < 2; ++i)
+    ctx->pool.run(n, n < (size_t(1) << 19) ? size_t(1) << 15 : size_t(1) << 18, [=](size_t i0, size_t i1) {
+        for (size_t i = i0; i < i1; i += 512) __atomic_fetch_add(reinterpret_cast<unsigned char*>(host + i), 0, __ATOMIC_RELAXED);
+        __atomic_fetch_add(reinterpret_cast<unsigned char*>(host + i1 - 1), 0, __ATOMIC_RELAXED);
+    });
+}
+
+int ensurePin(skgpu_ctx* ctx, size_t n)
+{
+    const size_t size = n <= (size_t(4) << 20) ? size_t(1) << 19 : n <= (size_t(16) << 20) ? size_t(2) << 20 : size_t(4) << 20;
+    if (ctx->pinDoubles < size)
     {
-        if (!ctx->pin[i]) CK(cudaMallocHost(reinterpret_cast<void**>(&ctx->pin[i]), PIN_DOUBLES * sizeof(double)));
-        if (!ctx->pinEv[i]) CK(cudaEventCreateWithFlags(&ctx->pinEv[i], cudaEventDisableTiming));
+        CK(cudaStreamSynchronize(ctx->stream));  // copies out of the present buffers
+        ctx->pinDoubles = 0;
+        for (double*& pin : ctx->pin)
+        {
+            if (pin) cudaFreeHost(pin);
+            pin = nullptr;
+        }
+        for (double*& pin : ctx->pin) CK(cudaMallocHost(reinterpret_cast<void**>(&pin), size * sizeof(double)));
+        ctx->pinDoubles = size;
+    }
+    for (cudaEvent_t& ev : ctx->pinEv)
+        if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    return SKGPU_OK;
+}
+
+// Copies n doubles of pageable host memory to the device through the same buffers (the driver's own
+// copy of pageable memory runs at 6 GB/s, this at the speed of the host's memory), in the context's
+// stream; the host array is read by the time it returns.
+int copyIn(skgpu_ctx* ctx, const double* host, size_t n, double* dev)
+{
+    if (n <= PLAIN_DOUBLES)
+    {
+        CK(cudaMemcpyAsync(dev, host, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+        return SKGPU_OK;
+    }
+    int rc = ensurePin(ctx, n);
+    if (rc) return rc;
+    const size_t pin = ctx->pinDoubles, chunks = (n + pin - 1) / pin;
+    for (size_t c = 0; c < chunks; ++c)
+    {
+        const size_t a = c * pin, len = std::min(pin, n - a);
+        // the copy out of the buffer two chunks before, or that of an earlier call
+        CK(cudaEventSynchronize(ctx->pinEv[c & 1]));
+        double* to = ctx->pin[c & 1];
+        ctx->pool.run(len, COPY_GRAIN, [=](size_t i0, size_t i1) { std::memcpy(to + i0, host + a + i0, (i1 - i0) * sizeof(double)); });
+        CK(cudaMemcpyAsync(dev + a, to, len * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+        CK(cudaEventRecord(ctx->pinEv[c & 1], ctx->stream));
     }
     return SKGPU_OK;
 }
 
-// Adds n doubles of device memory into a host array: chunked copies into two pinned buffers, the
-// copy of chunk c+1 in flight while the host cores add chunk c.
-int addInto(skgpu_ctx* ctx, const double* dev, size_t n, double* host)
+// Hands the chunks of n doubles of device memory to `take` (chunk's offset, its data, its length) as they
+// arrive in the buffers, the copy of chunk c+1 in flight meanwhile.
+int readOut(skgpu_ctx* ctx, const double* dev, size_t n, const std::function<void(size_t, const double*, size_t)>& take)
 {
-    if (!host || !dev || n == 0) return SKGPU_OK;
-    int rc = ensurePin(ctx);
+    int rc = ensurePin(ctx, n);
     if (rc) return rc;
-    const size_t chunks = (n + PIN_DOUBLES - 1) / PIN_DOUBLES;
+    const size_t pin = ctx->pinDoubles, chunks = (n + pin - 1) / pin;
     auto issue = [&](size_t c) {
-        const size_t a = c * PIN_DOUBLES, len = std::min(PIN_DOUBLES, n - a);
+        const size_t a = c * pin, len = std::min(pin, n - a);
         cudaError_t e = cudaMemcpyAsync(ctx->pin[c & 1], dev + a, len * sizeof(double), cudaMemcpyDeviceToHost,
                                         ctx->stream);
         return e == cudaSuccess ? cudaEventRecord(ctx->pinEv[c & 1], ctx->stream) : e;
@@ -220,36 +270,45 @@ int addInto(skgpu_ctx* ctx, const double* dev, size_t n, double* host)
     CK(issue(0));
     for (size_t c = 0; c < chunks; ++c)
     {
-        // buffer (c+1)&1 held chunk c-1, whose add finished in the previous iteration
+        // buffer (c+1)&1 held chunk c-1, which was taken in the previous iteration
         if (c + 1 < chunks) CK(issue(c + 1));
         CK(cudaEventSynchronize(ctx->pinEv[c & 1]));
-        double* to = host + c * PIN_DOUBLES;
-        const double* from = ctx->pin[c & 1];
-        ctx->pool.run(std::min(PIN_DOUBLES, n - c * PIN_DOUBLES), ADD_GRAIN, [=](size_t i0, size_t i1) {
-            for (size_t i = i0; i < i1; ++i) to[i] += from[i];
-        });
+        take(c * pin, ctx->pin[c & 1], std::min(pin, n - c * pin));
     }
     return SKGPU_OK;
 }
 
-// Copies n doubles of pageable host memory to the device through the same buffers (the driver's own
-// copy of pageable memory runs at 6 GB/s, this at the speed of the host's memory); returns when done.
-int copyIn(skgpu_ctx* ctx, const double* host, size_t n, double* dev)
+int copyOut(skgpu_ctx* ctx, const double* dev, size_t n, double* host)
 {
-    int rc = ensurePin(ctx);
-    if (rc) return rc;
-    const size_t chunks = (n + PIN_DOUBLES - 1) / PIN_DOUBLES;
-    for (size_t c = 0; c < chunks; ++c)
+    if (n <= PLAIN_DOUBLES)
     {
-        const size_t a = c * PIN_DOUBLES, len = std::min(PIN_DOUBLES, n - a);
-        if (c >= 2) CK(cudaEventSynchronize(ctx->pinEv[c & 1]));
-        double* to = ctx->pin[c & 1];
-        ctx->pool.run(len, COPY_GRAIN, [=](size_t i0, size_t i1) { std::memcpy(to + i0, host + a + i0, (i1 - i0) * sizeof(double)); });
-        CK(cudaMemcpyAsync(dev + a, to, len * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-        CK(cudaEventRecord(ctx->pinEv[c & 1], ctx->stream));
+        CK(cudaMemcpyAsync(host, dev, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        return SKGPU_OK;
     }
-    CK(cudaStreamSynchronize(ctx->stream));
-    return SKGPU_OK;
+    return readOut(ctx, dev, n, [&](size_t at, const double* from, size_t len) {
+        if (at == 0) mapPages(ctx, host, n);
+        ctx->pool.run(len, COPY_GRAIN, [=](size_t i0, size_t i1) { std::memcpy(host + at + i0, from + i0, (i1 - i0) * sizeof(double)); });
+    });
+}
+
+// adds n doubles of device memory into a host array
+int addInto(skgpu_ctx* ctx, const double* dev, size_t n, double* host)
+{
+    if (!host || !dev || n == 0) return SKGPU_OK;
+    if (n <= PLAIN_DOUBLES)
+    {
+        std::vector<double> v(n);
+        int rc = copyOut(ctx, dev, n, v.data());
+        for (size_t i = 0; i < n && !rc; ++i) host[i] += v[i];
+        return rc;
+    }
+    return readOut(ctx, dev, n, [&](size_t at, const double* from, size_t len) {
+        if (at == 0) mapPages(ctx, host, n);
+        ctx->pool.run(len, COPY_GRAIN, [=](size_t i0, size_t i1) {
+            for (size_t i = i0; i < i1; ++i) host[at + i] += from[i];
+        });
+    });
 }
 
 // out[m * nbins + ell] = in[ell * cells + m], through 32 x 32 shared-memory tiles (both sides coalesced)
@@ -286,17 +345,6 @@ __global__ void __launch_bounds__(256) finiteKernel(const double* __restrict__ v
          i += static_cast<size_t>(gridDim.x) * blockDim.x)
         ok = ok && isfinite(v[i]);
     if (!ok) *bad = 1;
-}
-
-void freeRays(skgpu_ctx* ctx)
-{
-    for (int i = 0; i < 2; ++i)
-    {
-        devFree(ctx->rayDev[i]);
-        if (ctx->rayPin[i]) cudaFreeHost(ctx->rayPin[i]);
-        ctx->rayPin[i] = nullptr;
-    }
-    ctx->rayBytes = 0;
 }
 
 template<typename T>
@@ -426,7 +474,7 @@ void skgpu_destroy(skgpu_ctx* ctx)
     devFree(ctx->rfEll);
     devFree(ctx->rf);
     devFree(ctx->srcBuf);
-    freeRays(ctx);
+    devFree(ctx->rayDev);
     freeWave(ctx);
     ctx->graphCache.release();
     for (void* p : ctx->batchBufs) cudaFree(p);
@@ -2447,64 +2495,6 @@ int skgpu_last_run_ms(skgpu_ctx* ctx, double* ms)
 // path segments
 // ------------------------------------------------------------------------------------------------
 
-// Takes rays through the device in chunks of at most 16 MB: `launch` runs on a chunk's rays and its
-// block of results (outBytes per ray), `store` hands the results on. Two chunks are in flight, each with
-// a device and a pinned block that the context keeps: while one is on the device, the host fills and
-// empties the other. Allocating per call and copying pageable memory took 120 of 180 us for a few
-// hundred rays, and 5 of 7 ms for 1e6.
-static cudaError_t rayChunks(skgpu_ctx* ctx, size_t n, const double* rays, size_t outBytes, int* errFlag,
-                             const std::function<cudaError_t(int, double*, unsigned char*)>& launch,
-                             const std::function<void(size_t, int, const unsigned char*)>& store)
-{
-    const size_t rayBytes = 6 * sizeof(double), perRay = rayBytes + outBytes;
-    const size_t rows = std::min(n, std::max<size_t>(1, (size_t(16) << 20) / perRay));
-    const size_t need = rows * perRay + sizeof(int);
-    cudaError_t e = cudaSuccess;
-    if (ctx->rayBytes < need)
-    {
-        freeRays(ctx);
-        const size_t bytes = std::max<size_t>(need, size_t(1) << 18);
-        for (int i = 0; i < 2 && e == cudaSuccess; ++i)
-        {
-            e = devAlloc(&ctx->rayDev[i], bytes);
-            if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&ctx->rayPin[i]), bytes);
-        }
-        if (e == cudaSuccess) ctx->rayBytes = bytes;
-    }
-    for (int i = 0; i < 2 && e == cudaSuccess; ++i)
-        if (!ctx->pinEv[i]) e = cudaEventCreateWithFlags(&ctx->pinEv[i], cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaMemsetAsync(ctx->errFlag, 0, sizeof(int), ctx->stream);
-    const size_t chunks = (n + rows - 1) / rows;
-    auto size = [&](size_t c) { return static_cast<int>(std::min(rows, n - c * rows)); };
-    auto finish = [&](size_t c) {
-        cudaError_t r = cudaEventSynchronize(ctx->pinEv[c & 1]);
-        const unsigned char* out = ctx->rayPin[c & 1] + size(c) * rayBytes;
-        if (r == cudaSuccess) store(c * rows, size(c), out);
-        if (r == cudaSuccess) std::memcpy(errFlag, out + size(c) * outBytes, sizeof(int));
-        return r;
-    };
-    for (size_t c = 0; c < chunks && e == cudaSuccess; ++c)
-    {
-        const int k = size(c);
-        unsigned char *dev = ctx->rayDev[c & 1], *pin = ctx->rayPin[c & 1];
-        const double* from = rays + 6 * c * rows;
-        double* to = reinterpret_cast<double*>(pin);
-        ctx->pool.run(6 * static_cast<size_t>(k), COPY_GRAIN,
-                      [=](size_t i0, size_t i1) { std::memcpy(to + i0, from + i0, (i1 - i0) * sizeof(double)); });
-        e = cudaMemcpyAsync(dev, pin, k * rayBytes, cudaMemcpyHostToDevice, ctx->stream);
-        if (e == cudaSuccess) e = launch(k, reinterpret_cast<double*>(dev), dev + k * rayBytes);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(pin + k * rayBytes, dev + k * rayBytes, k * outBytes, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(pin + k * perRay, ctx->errFlag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(ctx->pinEv[c & 1], ctx->stream);
-        if (e == cudaSuccess && c > 0) e = finish(c - 1);
-    }
-    if (e == cudaSuccess) e = finish(chunks - 1);
-    if (e != cudaSuccess) cudaStreamSynchronize(ctx->stream);  // nothing in flight uses the blocks any more
-    return e;
-}
-
 int skgpu_trace_paths(skgpu_ctx* ctx, int32_t num_rays, const double* rays, int32_t max_segments, int32_t precision,
                       int32_t* count, int32_t* m, double* ds)
 {
@@ -2515,29 +2505,25 @@ int skgpu_trace_paths(skgpu_ctx* ctx, int32_t num_rays, const double* rays, int3
     if (precision != SKGPU_PREC_FP64_EXACT && precision != SKGPU_PREC_FP32) return fail(ctx, SKGPU_ERR_ARG, "trace: bad precision");
     if (num_rays == 0) return SKGPU_OK;
     CK(cudaSetDevice(ctx->device));
-    // a ray's share of a chunk: the ray, its count, cells and lengths (the entries past its count are 0)
-    const size_t seg = max_segments;
+    size_t n = num_rays, ns = n * static_cast<size_t>(max_segments);
+    double *dRays = nullptr, *dDs = nullptr;
+    int *dCount = nullptr, *dM = nullptr;
+    auto cleanup = [&]() { devFree(dRays); devFree(dDs); devFree(dCount); devFree(dM); };
+    cudaError_t e = devUpload(&dRays, rays, 6 * n);
+    if (e == cudaSuccess) e = devAlloc(&dDs, ns);
+    if (e == cudaSuccess) e = devAlloc(&dCount, n);
+    if (e == cudaSuccess) e = devAlloc(&dM, ns);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ctx->errFlag, 0, sizeof(int), ctx->stream);
+    if (e == cudaSuccess)
+        e = (precision == SKGPU_PREC_FP32 ? launchTracePathsFP32 : launchTracePathsFP64)(
+            precision, ctx->g, num_rays, dRays, max_segments, dCount, dM, dDs, ctx->errFlag, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     int errFlag = 0;
-    cudaError_t e = rayChunks(
-        ctx, num_rays, rays, sizeof(int) + seg * (sizeof(int) + sizeof(double)), &errFlag,
-        [&](int k, double* dRays, unsigned char* out) {
-            double* dDs = reinterpret_cast<double*>(out);
-            int* dM = reinterpret_cast<int*>(dDs + k * seg);
-            int* dCount = dM + k * seg;
-            cudaError_t r = cudaMemsetAsync(out, 0, k * (sizeof(int) + seg * (sizeof(int) + sizeof(double))), ctx->stream);
-            if (r != cudaSuccess) return r;
-            return (precision == SKGPU_PREC_FP32 ? launchTracePathsFP32 : launchTracePathsFP64)(
-                precision, ctx->g, k, dRays, max_segments, dCount, dM, dDs, ctx->errFlag, ctx->stream);
-        },
-        [&](size_t first, int k, const unsigned char* out) {
-            const double* hDs = reinterpret_cast<const double*>(out);
-            const int* hM = reinterpret_cast<const int*>(hDs + k * seg);
-            std::memcpy(count + first, hM + k * seg, k * sizeof(int));
-            ctx->pool.run(k * seg, COPY_GRAIN, [&](size_t i0, size_t i1) {
-                std::memcpy(ds + first * seg + i0, hDs + i0, (i1 - i0) * sizeof(double));
-                std::memcpy(m + first * seg + i0, hM + i0, (i1 - i0) * sizeof(int));
-            });
-        });
+    if (e == cudaSuccess) e = cudaMemcpy(&errFlag, ctx->errFlag, sizeof(int), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(count, dCount, n * sizeof(int), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(m, dM, ns * sizeof(int), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(ds, dDs, ns * sizeof(double), cudaMemcpyDeviceToHost);
+    cleanup();
     if (e == cudaErrorNotSupported) return fail(ctx, SKGPU_ERR_UNSUPPORTED, "trace: no walker of this precision for the grid kind");
     if (e != cudaSuccess) return fail(ctx, SKGPU_ERR_CUDA, std::string("trace: ") + cudaGetErrorString(e));
     if (errFlag) return fail(ctx, SKGPU_ERR_TIMEOUT, "trace: a path exceeded its segment guard");
@@ -2555,15 +2541,28 @@ int skgpu_optical_depths(skgpu_ctx* ctx, int32_t num_rays, const double* rays, d
     if (num_rays == 0) return SKGPU_OK;
     // DustMix::sectionExt(lambda) = sigma_ext[locateClip(lambda borders, lambda)]
     double section = ctx->mixExtHost[std::max(0, skg::locateClip(ctx->mixLbHost.data(), ctx->nmix, lambda))];
-    int errFlag = 0;
-    cudaError_t e = rayChunks(
-        ctx, num_rays, rays, sizeof(double), &errFlag,
-        [&](int k, double* dRays, unsigned char* out) {
-            return (precision == SKGPU_PREC_FP32 ? launchOpticalDepthsFP32 : launchOpticalDepthsFP64)(
-                precision, ctx->g, ctx->dens, section, k, dRays, reinterpret_cast<double*>(out), ctx->errFlag, ctx->stream);
-        },
-        [&](size_t first, int k, const unsigned char* out) { std::memcpy(tau + first, out, k * sizeof(double)); });
-    if (e != cudaSuccess) return fail(ctx, SKGPU_ERR_CUDA, std::string("optical depths: ") + cudaGetErrorString(e));
+    // rays and depths in device memory that the context keeps, at most 32 MB of it; a larger number of rays
+    // goes through it in parts
+    const size_t perRay = 7 * sizeof(double), rows = std::min<size_t>(num_rays, (size_t(32) << 20) / perRay);
+    if (ctx->rayRows < rows)
+    {
+        devFree(ctx->rayDev);
+        ctx->rayRows = 0;
+        CK(devAlloc(&ctx->rayDev, 7 * rows));
+        ctx->rayRows = rows;
+    }
+    double *dRays = ctx->rayDev, *dTau = dRays + 6 * rows;
+    CK(cudaMemsetAsync(ctx->errFlag, 0, sizeof(int), ctx->stream));
+    for (size_t first = 0; first < static_cast<size_t>(num_rays); first += rows)
+    {
+        const int k = static_cast<int>(std::min(rows, num_rays - first));
+        int rc = copyIn(ctx, rays + 6 * first, 6 * static_cast<size_t>(k), dRays);
+        if (rc) return rc;
+        cudaError_t e = (precision == SKGPU_PREC_FP32 ? launchOpticalDepthsFP32 : launchOpticalDepthsFP64)(
+            precision, ctx->g, ctx->dens, section, k, dRays, dTau, ctx->errFlag, ctx->stream);
+        if (e != cudaSuccess) return fail(ctx, SKGPU_ERR_CUDA, std::string("optical depths: ") + cudaGetErrorString(e));
+        if ((rc = copyOut(ctx, dTau, k, tau + first))) return rc;
+    }
     return SKGPU_OK;
 }
 

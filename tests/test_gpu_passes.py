@@ -5,7 +5,7 @@
   by the order of their FP64 additions (1e-12 of the largest entry; a bin sums at most 1e4 terms of
   one sign, whose rounding errors stay below 1e4 x 1.1e-16).
 - Statistics buffers that a run left behind serve a later run with more slots.
-- Rays in any number, around the chunks of the path entry points, give what one ray at a time gives.
+- Rays in any number, around the parts in which their depths are taken, give what a few give.
 - A radiation field comes back as it was uploaded, and one with a non-finite value changes nothing.
 """
 import numpy as np
@@ -90,9 +90,10 @@ def test_statistics_buffers_of_growing_runs(golden, gpu_backend, oracle_backend)
             assert np.array_equal(x["stats"][0], y["stats"][0])
 
 
-@pytest.mark.parametrize("n", [1, 2, 299592, 299593, 299594, 600001])
-def test_optical_depths_in_chunks(golden, gpu_backend, n):
-    """16 MB hold 299 593 rays of 56 bytes."""
+@pytest.mark.parametrize("n", [1, 2, 1365, 1366, 87381, 87382, 599186, 599187, 1200001])
+def test_optical_depths_in_parts(golden, gpu_backend, n):
+    """Around the direct copies (64 KB: 1 365 rays of 48 bytes), the 4 MB chunks of the pinned ones (87 381)
+    and the device block (32 MB: 599 186 rays of 56 bytes)."""
     z = golden("paths_cartesian_c16.npz")
     sc = Scene.from_export(z)
     sc.upload(gpu_backend)
@@ -100,21 +101,6 @@ def test_optical_depths_in_chunks(golden, gpu_backend, n):
     few = gpu_backend.optical_depths(rays, 0.55e-6)
     at = np.arange(n) % len(rays)
     assert np.array_equal(gpu_backend.optical_depths(rays[at], 0.55e-6), few[at])
-
-
-@pytest.mark.parametrize("n,segments", [(1, 64), (400, 64), (21000, 64), (3, 700000)])
-def test_path_segments_in_chunks(golden, gpu_backend, n, segments):
-    """16 MB hold 20 460 rays of 64 segments, and one of 700 000."""
-    z = golden("paths_cartesian_c16.npz")
-    Scene.from_export(z).upload(gpu_backend)
-    rays = z["rays"]
-    count, m, ds = gpu_backend.trace_paths(rays, 64)
-    at = np.arange(n) % len(rays)
-    c, mm, dd = gpu_backend.trace_paths(rays[at], segments)
-    assert np.array_equal(c, count[at])
-    w = min(64, segments)
-    assert np.array_equal(mm[:, :w], m[at]) and np.array_equal(dd[:, :w], ds[at])
-    assert not mm[:, w:].any() and not dd[:, w:].any()
 
 
 @pytest.mark.parametrize("bins", [1, 31, 32, 33, 70])
