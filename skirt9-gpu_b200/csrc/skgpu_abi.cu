@@ -11,11 +11,13 @@
 #include <mutex>
 #include <type_traits>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <limits>
 #include <string>
 #include <thread>
 #include <vector>
+#include <sys/mman.h>
 
 #include "../../include/skgpu.h"
 #include "internal.hpp"
@@ -188,8 +190,7 @@ void freeWave(skgpu_ctx* ctx)
 
 // Pinned staging buffers, two of 4 MB for arrays of up to 32 MB, of 16 MB up to 128 MB, of 32 MB above: a
 // chunk's copy and the host's work on another overlap, and a context pays for pinned memory what its
-// arrays are worth (0.8 ms per MB; two of 64 MB from the first fetch on made a first pass 100 ms longer).
-// Arrays of up to 64 KB go without.
+// arrays are worth. Arrays of up to 64 KB go without.
 constexpr size_t PLAIN_DOUBLES = size_t(1) << 13;
 
 // Doubles that a host core takes at least (0.5 MB).
@@ -208,6 +209,26 @@ void mapPages(skgpu_ctx* ctx, double* host, size_t n)
     });
 }
 
+void freePin(double* pin)
+{
+    if (cudaHostUnregister(pin) != cudaSuccess) cudaGetLastError();  // one that could not be pinned
+    std::free(pin);
+}
+
+// Pins a large page at a time: 0.8 ms for 4 MB and 4.0 ms for 32 MB, where cudaMallocHost takes 2.6 and
+// 13.4 ms, with the same copy rate (50 and 56 GB/s). Memory that cannot be pinned serves too, only slower.
+double* allocPin(size_t doubles)
+{
+    constexpr size_t PAGE = size_t(2) << 20;
+    const size_t bytes = doubles * sizeof(double);  // a multiple of a large page
+    void* pin = std::aligned_alloc(PAGE, bytes);
+    if (!pin) return nullptr;
+    madvise(pin, bytes, MADV_HUGEPAGE);
+    for (size_t i = 0; i < bytes; i += 4096) static_cast<volatile char*>(pin)[i] = 0;
+    if (cudaHostRegister(pin, bytes, cudaHostRegisterDefault) != cudaSuccess) cudaGetLastError();
+    return static_cast<double*>(pin);
+}
+
 int ensurePin(skgpu_ctx* ctx, size_t n)
 {
     const size_t size = n <= (size_t(4) << 20) ? size_t(1) << 19 : n <= (size_t(16) << 20) ? size_t(2) << 20 : size_t(4) << 20;
@@ -217,10 +238,10 @@ int ensurePin(skgpu_ctx* ctx, size_t n)
         ctx->pinDoubles = 0;
         for (double*& pin : ctx->pin)
         {
-            if (pin) cudaFreeHost(pin);
-            pin = nullptr;
+            if (pin) freePin(pin);
+            pin = allocPin(size);
         }
-        for (double*& pin : ctx->pin) CK(cudaMallocHost(reinterpret_cast<void**>(&pin), size * sizeof(double)));
+        if (!ctx->pin[0] || !ctx->pin[1]) return fail(ctx, SKGPU_ERR_CUDA, "no host memory for the staging buffers");
         ctx->pinDoubles = size;
     }
     for (cudaEvent_t& ev : ctx->pinEv)
@@ -489,7 +510,7 @@ void skgpu_destroy(skgpu_ctx* ctx)
     if (ctx->doneHost) cudaFreeHost(ctx->doneHost);
     for (int i = 0; i < 2; ++i)
     {
-        if (ctx->pin[i]) cudaFreeHost(ctx->pin[i]);
+        if (ctx->pin[i]) freePin(ctx->pin[i]);
         if (ctx->pinEv[i]) cudaEventDestroy(ctx->pinEv[i]);
     }
     if (ctx->timerEvents)
