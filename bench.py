@@ -454,7 +454,7 @@ def traversal_times(be, step, steps):
 def result_line(args, name, world, value, total_ms, trace_ms, trace_launches, counters, kind, prec, clk, e2e,
                 per_gpu):
     """The JSON line of our arm; the roofline is that of the traversal kernel: its algorithmic bytes per
-    launch over its average launch duration (CUDA events on the launch stream, timed steps)."""
+    launch over its average launch duration (CUDA events on the launch stream, in one extra step of plain passes)."""
     from skgpu import abi
     peak, peak_kind = peaks()
     trace_bytes_per_launch = trace_algorithmic_bytes(counters, kind) / max(1, trace_launches / args.steps)
