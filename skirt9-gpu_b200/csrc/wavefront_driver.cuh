@@ -17,7 +17,7 @@ struct WaveLaunch
 {
     int traceBlocks, shadeBlocks, guideBlocks, threads;
     bool guided, multi;
-    // pipelined passes: whether detections come before the step that may end their history, whether
+    // pipelined passes: whether detections come before the step that may end their history (pilots), whether
     // any scene forces its scattering, and the second stream with its events
     bool pipelined, strict, forced;
     int peelBlocks, forcedBlocks, searchBlocks;
@@ -50,11 +50,12 @@ void launchTrace(const Wave& w, int cur, int blocks, const WaveLaunch& L, cudaSt
 // The passes of a captured graph without stage timing, on two streams:
 //   main  traversal of the complete forced paths, sampling of their interaction depths, traversal of
 //         the searches for the interaction points, then the step (interactions, new histories)
-//   side  traversal of the peel-off rays that the previous step queued, then their detection
+//   side  statistics of the histories that the previous step ended, traversal of the peel-off rays that it
+//         queued, then their detection
 // One pass carries a packet from one interaction to the next. A peel-off task holds what it needs of
 // its packet, so the packet goes on meanwhile: the side stream may lag by a pass, and the last long
-// rays of one traversal run beside the next one instead of alone. Only where the statistics or the
-// pilot records of a history are closed at its end do its detections come first (`strict`).
+// rays of one traversal run beside the next one instead of alone. Only where the pilot records of a
+// history are closed at its end do its detections come first (`strict`).
 // The plain pass below walks the forced paths and the searches in passes of their own (twice the
 // passes, each as long as its longest ray), joins its streams in each, and takes eight kernels.
 template<class Walker>
@@ -70,8 +71,11 @@ cudaError_t enqueuePipelined(const Wave& w, int pass, const WaveLaunch& L, cudaS
         shadeProp1Kernel<<<L.shadeBlocks, L.threads, 0, s>>>(w, cur, cur);
     }
     launchTrace<Walker, TRACE_SEARCH>(w, cur, L.searchBlocks, L, s);
-    // the step refills the peel-off queue that the side stream emptied in the previous pass
-    if (!L.strict && pass > 0 && (e = cudaStreamWaitEvent(s, L.join, 0)) != cudaSuccess) return e;
+    // the step refills the peel-off queue that the side stream emptied in the previous pass, and launches
+    // into the slots whose statistics it has taken (of a graph's first pass: those of the graph before)
+    if (w.anyStats) flushEndedKernel<<<L.shadeBlocks, L.threads, 0, L.side>>>(w, nxt);
+    if ((e = cudaEventRecord(L.join, L.side)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(s, L.join, 0)) != cudaSuccess) return e;
     launchTrace<Walker, TRACE_PEEL>(w, cur, L.peelBlocks, L, L.side);
     shadePeelKernel<<<L.shadeBlocks, L.threads, 0, L.side>>>(w, cur);
     if ((e = cudaEventRecord(L.join, L.side)) != cudaSuccess) return e;
@@ -196,7 +200,7 @@ cudaError_t runWave(const Wave& wave, int numSMs, cudaStream_t s, unsigned long 
     if (useGraph && cache && !timer && pipelinedPasses() && cache->ensureSide() == cudaSuccess)
     {
         L.pipelined = true;
-        L.strict = w.anyStats || w.sc.guideMode == 1;
+        L.strict = w.sc.guideMode == 1;
         L.forced = w.nScenes > 1 || w.sc.forced;
         const int cap = w.traceBlocksPerSM > 0 ? w.traceBlocksPerSM : 1 << 30;
         const size_t smem = traceSmemBytes(w);
@@ -216,7 +220,7 @@ cudaError_t runWave(const Wave& wave, int numSMs, cudaStream_t s, unsigned long 
         cudaError_t ea = cudaFuncSetAttribute(guideScatterKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GM_SMEM_BYTES);
         if (ea != cudaSuccess) return ea;
     }
-    if (cache) cache->kernelsPerPass = (L.pipelined ? (L.forced ? 6 : 4) + (L.guided ? 1 : 0) : 7) + (L.guided ? 1 : 0);
+    if (cache) cache->kernelsPerPass = (L.pipelined ? (L.forced ? 6 : 4) + (L.guided ? 1 : 0) + (w.anyStats ? 1 : 0) : 7) + (L.guided ? 1 : 0);
     initPoolKernel<<<L.shadeBlocks, L.threads, 0, s>>>(w, w.anyStats && clearStats ? 1 : 0);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -289,6 +293,12 @@ cudaError_t runWave(const Wave& wave, int numSMs, cudaStream_t s, unsigned long 
             e = cudaErrorLaunchTimeout;
             break;
         }
+    }
+    if (e == cudaSuccess && L.pipelined && w.anyStats)
+    {
+        flushEndedKernel<<<L.shadeBlocks, L.threads, 0, s>>>(w, 1);  // the histories that the last pass ended
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     }
     if (exec && !(cache && cache->exec == exec)) cudaGraphExecDestroy(exec);
     if (cache && e != cudaSuccess) cache->reset();  // after an error the next run captures afresh
