@@ -56,10 +56,14 @@ def test_pipelined_equals_plain_passes(golden, gpu_backend, name, stats, forced,
     assert_same(a, b)
 
 
+@pytest.mark.parametrize("stats", [0, 1])
 @pytest.mark.parametrize("slots", [256, 1000])
-def test_pipelined_passes_refill_a_small_pool(golden, gpu_backend, slots):
-    """More histories than slots: every slot is freed and launched into again many times."""
+def test_pipelined_passes_refill_a_small_pool(golden, gpu_backend, slots, stats):
+    """More histories than slots: every slot is freed and launched into again many times, its statistics
+    taken in between."""
     sc = Scene.from_export(golden("shell_c16.npz"))
+    for ins in sc.instruments:
+        ins["stats"] = stats
     sc.upload(gpu_backend)
     a = sc.run(gpu_backend, 30001, seed=2, precision=abi.PREC_FP32)
     abi.set_launch_shape(gpu_backend, slots)
