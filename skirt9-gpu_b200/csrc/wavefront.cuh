@@ -322,8 +322,12 @@ __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __g
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int refillMin = w.refillMin > 0 ? w.refillMin : Walker::kRefillMin;
-    unsigned n0 = w.ctl->qn[cur][0], n1 = w.ctl->qn[cur][1], n2 = w.ctl->qn[cur][2], n3 = w.ctl->qn[cur][3];
-    const unsigned total = Mode == TRACE_PEEL ? n0 : Mode == TRACE_FORCED ? n1 : Mode == TRACE_SEARCH ? n2 + n3 : n0 + n1 + n2 + n3;
+    // the tasks of the kinds that this launch walks; the counts of the others are not read, since the kernels
+    // that empty those queues may run beside this one (pipelined passes)
+    auto tasks = [&](int k, int mode) { return Mode == TRACE_ALL || Mode == mode ? w.ctl->qn[cur][k] : 0u; };
+    const unsigned n0 = tasks(K_PEEL, TRACE_PEEL), n1 = tasks(K_PROP1, TRACE_FORCED), n2 = tasks(K_PROP2, TRACE_SEARCH),
+                   n3 = tasks(K_FREE, TRACE_SEARCH);
+    const unsigned total = n0 + n1 + n2 + n3;
     if (total == 0) return;
     unsigned* const cursor = Mode == TRACE_FORCED   ? &w.ctl->forcedCursor
                              : Mode == TRACE_SEARCH ? &w.ctl->searchCursor
@@ -374,8 +378,6 @@ __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __g
                 }
                 else
                 {
-                    if (Mode == TRACE_FORCED) t += n0;
-                    if (Mode == TRACE_SEARCH) t += n0 + n1;
                     if (Mode == TRACE_PEEL || (Mode == TRACE_ALL && t < n0)) { kind = K_PEEL; idx = t; }
                     else if (Mode == TRACE_FORCED || (Mode == TRACE_ALL && t < n0 + n1)) { kind = K_PROP1; idx = t - n0; }
                     else if (t < n0 + n1 + n2) { kind = K_PROP2; idx = t - n0 - n1; }

@@ -56,6 +56,75 @@ def test_pipelined_equals_plain_passes(golden, gpu_backend, name, stats, forced,
     assert_same(a, b)
 
 
+def assert_passes_agree(be, run):
+    """The run's pipelined and plain passes: counters and tallies; returns both results. (stats_spilled is no such
+    counter: which keys get the last places of a slot's buffer depends on timing in either form.)"""
+    a, b = run(), timed(be, run)
+    for key in ("histories", "crossings", "scatterings", "peel_detections", "rf_stores"):
+        assert a.counters[key] == b.counters[key], key
+    assert_same(a, b)
+    return a, b
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64_EXACT, abi.PREC_FP32])
+@pytest.mark.parametrize("forced", [True, False])
+@pytest.mark.parametrize("n", [1, 333, 20000])
+def test_pipelined_equals_plain_passes_of_tetrahedra(golden, gpu_backend, forced, precision, n):
+    """Queues of every relative length beside one another: the searches of a pass run while the peel-off
+    queue of the same pass is walked and emptied."""
+    sc = Scene.from_export(golden("stats_tetra.npz"))
+    sc.force_scattering = forced
+    sc.upload(gpu_backend)
+    assert_passes_agree(gpu_backend, lambda: sc.run(gpu_backend, n, seed=6, precision=precision))
+
+
+@pytest.mark.parametrize("n", [1, 333, 20000])
+def test_pipelined_equals_plain_passes_of_pilots(golden, gpu_backend, n):
+    """Pilot records take the detections of a history before the step that ends it."""
+    sc = Scene.from_export(golden("shell_c16.npz"))
+    sc.upload(gpu_backend)
+    abi.guide_init(gpu_backend, None, 1)
+    records = []
+
+    def run():
+        abi.guide_set_mode(gpu_backend, abi.GUIDE_RECORD, 0, 0.0, 1.0, 1 << 20)  # starts the records anew
+        res = sc.run(gpu_backend, n, seed=3, precision=abi.PREC_FP32)
+        rec = abi.guide_records(gpu_backend)
+        records.append(rec[np.lexsort(rec[:, :11].T)])  # by inputs and direction: the order of the events is free
+        return res
+
+    assert_passes_agree(gpu_backend, run)
+    a, b = records
+    assert np.array_equal(a[:, :11], b[:, :11]) and np.array_equal(a[:, 12], b[:, 12])
+    # what follows an event is a difference of FP64 sums of at most 1e4 detections, kept in FP32
+    assert np.allclose(a[:, 11], b[:, 11], rtol=1e-6, atol=1e-10 * max(a[:, 11].max(initial=0), 1e-300))
+
+
+@pytest.mark.parametrize("n", [1, 333, 20000])
+def test_pipelined_equals_plain_passes_of_guided_runs(golden, gpu_backend, n):
+    """Guided scattering: the network's outputs for an event do not depend on the other events of its tile."""
+    sc = Scene.from_export(golden("shell_c16.npz"))
+    sc.upload(gpu_backend)
+    abi.guide_init(gpu_backend, None, 5)
+    abi.guide_set_mode(gpu_backend, abi.GUIDE_SAMPLE, 0, 0.5)
+    a, _ = assert_passes_agree(gpu_backend, lambda: sc.run(gpu_backend, n, seed=4, precision=abi.PREC_FP32))
+    assert n < 333 or a.counters["scatterings"] > 0
+
+
+def test_pipelined_equals_plain_passes_of_spilled_statistics(golden, gpu_backend):
+    """Histories with more keys than a slot buffers, taken on the side stream: 16 frames, albedo 0.95."""
+    sc = Scene.from_export(golden("shell_c16.npz"))
+    frame, sc.instruments = dict(sc.instruments[0], stats=1, same_observer=0), []
+    for th in np.radians(np.linspace(5, 175, 16)):
+        sc.instruments.append(dict(frame, kobs=(np.sin(th), 0.0, np.cos(th)),
+                                   trig=(np.cos(th), np.sin(th), 1.0, 0.0, 1.0, 0.0)))
+    sc.mix = dict(sc.mix, sigma_sca=0.95 * np.asarray(sc.mix["sigma_ext"]))
+    sc.min_weight_reduction = 1e8
+    sc.upload(gpu_backend)
+    a, _ = assert_passes_agree(gpu_backend, lambda: sc.run(gpu_backend, 2000, seed=23))
+    assert a.counters["stats_spilled"] > 0 and a.counters["stats_overflows"] == 0
+
+
 @pytest.mark.parametrize("stats", [0, 1])
 @pytest.mark.parametrize("slots", [256, 1000])
 def test_pipelined_passes_refill_a_small_pool(golden, gpu_backend, slots, stats):
