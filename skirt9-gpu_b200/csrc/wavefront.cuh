@@ -420,6 +420,8 @@ __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __g
                             fB = 0.;
                             fC = 0.;
                             iA = -1;
+                            // an empty forced path has nothing to search for: the step ends its history
+                            if (Mode == TRACE_SEARCH && fA < 0) kind = -1;
                         }
                     }
                 }

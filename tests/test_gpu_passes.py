@@ -78,6 +78,22 @@ def test_pipelined_equals_plain_passes_of_tetrahedra(golden, gpu_backend, forced
     assert_passes_agree(gpu_backend, lambda: sc.run(gpu_backend, n, seed=6, precision=precision))
 
 
+@pytest.mark.parametrize("precision", [abi.PREC_FP64_EXACT, abi.PREC_FP32])
+@pytest.mark.parametrize("explicit", [False, True])
+def test_pipelined_equals_plain_passes_of_empty_paths(golden, gpu_backend, explicit, precision):
+    """Forced paths of zero optical depth, through empty cells only or (explicit absorption) without scattering,
+    end their histories without a search: both forms count the same crossings."""
+    sc = Scene.from_export(golden("shell_c16.npz"))
+    sc.explicit_absorption = explicit
+    if explicit:
+        sc.mix = dict(sc.mix, sigma_sca=0.0 * np.asarray(sc.mix["sigma_ext"]))
+    else:
+        sc.density = np.where(np.arange(len(sc.density)) < len(sc.density) // 2, 0.0, sc.density)
+    sc.upload(gpu_backend)
+    a, _ = assert_passes_agree(gpu_backend, lambda: sc.run(gpu_backend, 5000, seed=8, precision=precision))
+    assert a.counters["scatterings"] == 0 if explicit else a.counters["scatterings"] > 0
+
+
 @pytest.mark.parametrize("n", [1, 333, 20000])
 def test_pipelined_equals_plain_passes_of_pilots(golden, gpu_backend, n):
     """Pilot records take the detections of a history before the step that ends it."""
