@@ -85,9 +85,9 @@ struct skgpu_ctx
     size_t pinDoubles = 0;
     cudaEvent_t pinEv[2] = {nullptr, nullptr};
     skg::HostPool pool;
-    // rays and results of skgpu_optical_depths: 7 doubles per row
-    double* rayDev = nullptr;
-    size_t rayRows = 0;
+    // device block of the calls that work in parts (rays and depths, a field on its way to the tally)
+    double* part = nullptr;
+    size_t partDoubles = 0;
 
     // launch shape set by skgpu_set_launch_shape (0: defaults)
     int shapePool = 0, shapeTraceBlocks = 0, shapeShadeBlocks = 0, shapeRefill = 0;

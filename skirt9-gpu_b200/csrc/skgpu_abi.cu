@@ -6,6 +6,7 @@
 // Voronoi nearest-site search and a uniform grid of tetrahedron bounding boxes for the tetra
 // cell search.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <functional>
 #include <mutex>
@@ -332,8 +333,8 @@ int addInto(skgpu_ctx* ctx, const double* dev, size_t n, double* host)
     });
 }
 
-// out[m * nbins + ell] = in[ell * cells + m], through 32 x 32 shared-memory tiles (both sides coalesced)
-__global__ void rfTransposeKernel(const double* __restrict__ in, double* __restrict__ out, int cells, int nbins)
+// out[m * ld + ell] = in[ell * cells + m], through 32 x 32 shared-memory tiles (both sides coalesced)
+__global__ void rfTransposeKernel(const double* __restrict__ in, double* __restrict__ out, int cells, int nbins, int ld)
 {
     __shared__ double tile[32][33];
     const int across = (cells + 31) / 32;
@@ -347,25 +348,40 @@ __global__ void rfTransposeKernel(const double* __restrict__ in, double* __restr
     for (int j = threadIdx.y; j < 32; j += blockDim.y)
     {
         int m = m0 + j, e = e0 + threadIdx.x;
-        if (e < nbins && m < cells) out[static_cast<size_t>(m) * nbins + e] = tile[threadIdx.x][j];
+        if (e < nbins && m < cells) out[static_cast<size_t>(m) * ld + e] = tile[threadIdx.x][j];
     }
 }
 
-cudaError_t transposeField(const double* in, double* out, int cells, int nbins, cudaStream_t s)
+cudaError_t transposeField(const double* in, double* out, int cells, int nbins, int ld, cudaStream_t s)
 {
     const size_t tiles = static_cast<size_t>((cells + 31) / 32) * ((nbins + 31) / 32);
-    rfTransposeKernel<<<static_cast<unsigned>(tiles), dim3(32, 8), 0, s>>>(in, out, cells, nbins);
+    rfTransposeKernel<<<static_cast<unsigned>(tiles), dim3(32, 8), 0, s>>>(in, out, cells, nbins, ld);
     return cudaGetLastError();
 }
 
-// sets *bad when a value is not finite
-__global__ void __launch_bounds__(256) finiteKernel(const double* __restrict__ v, size_t n, int* bad)
+// whether a large host array holds finite values only
+bool finiteLarge(skgpu_ctx* ctx, const double* v, size_t n)
 {
-    bool ok = true;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x)
-        ok = ok && isfinite(v[i]);
-    if (!ok) *bad = 1;
+    std::atomic<bool> ok{true};
+    ctx->pool.run(n, COPY_GRAIN, [&](size_t i0, size_t i1) {
+        bool good = true;
+        for (size_t i = i0; i < i1; ++i) good &= std::isfinite(v[i]);
+        if (!good) ok = false;
+    });
+    return ok;
+}
+
+// A device block that the context keeps for what passes through it in parts: at most 32 MB of it (or what a
+// single item takes).
+constexpr size_t PART_DOUBLES = size_t(4) << 20;
+int ensurePart(skgpu_ctx* ctx, size_t n)
+{
+    if (ctx->partDoubles >= n) return SKGPU_OK;
+    devFree(ctx->part);
+    ctx->partDoubles = 0;
+    CK(devAlloc(&ctx->part, n));
+    ctx->partDoubles = n;
+    return SKGPU_OK;
 }
 
 template<typename T>
@@ -495,7 +511,7 @@ void skgpu_destroy(skgpu_ctx* ctx)
     devFree(ctx->rfEll);
     devFree(ctx->rf);
     devFree(ctx->srcBuf);
-    devFree(ctx->rayDev);
+    devFree(ctx->part);
     freeWave(ctx);
     ctx->graphCache.release();
     for (void* p : ctx->batchBufs) cudaFree(p);
@@ -1967,44 +1983,28 @@ int skgpu_upload_radiation_field(skgpu_ctx* ctx, const double* rf)
     if (!rf) return fail(ctx, SKGPU_ERR_ARG, "radiation field: missing array");
     if (!ctx->nrf || !ctx->numCells) return fail(ctx, SKGPU_ERR_STATE, "radiation field: no medium or RF grid uploaded");
     CK(cudaSetDevice(ctx->device));
-    // The caller's layout is cell-major (m * nbins + ell), the device tally wavelength-major. The device
-    // checks the values and turns the layout: on the host the two took 19 of 21 ms for 8.6e4 cells and
-    // 50 bins, of which 34 MB are left to copy. Nothing of the context changes before the check.
-    const size_t len = static_cast<size_t>(ctx->numCells) * ctx->nrf;
-    const bool fits = ctx->rfLen == len;
-    double *raw = fits ? ctx->rfT : nullptr, *tally = fits ? ctx->rf : nullptr;
-    cudaError_t e = cudaSuccess;
-    if (!raw) e = devAlloc(&raw, len);
-    if (e == cudaSuccess && !tally) e = devAlloc(&tally, len);
-    auto giveBack = [&]() {
-        if (raw && raw != ctx->rfT) cudaFree(raw);
-        if (tally && tally != ctx->rf) cudaFree(tally);
-    };
-    int rc = SKGPU_OK, bad = 0;
-    if (e == cudaSuccess) rc = copyIn(ctx, rf, len, raw);
-    if (e == cudaSuccess && !rc) e = cudaMemsetAsync(ctx->errFlag, 0, sizeof(int), ctx->stream);
-    if (e == cudaSuccess && !rc)
-    {
-        finiteKernel<<<ctx->numSMs * 8, 256, 0, ctx->stream>>>(raw, len, ctx->errFlag);
-        e = cudaMemcpyAsync(&bad, ctx->errFlag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-    }
-    if (e == cudaSuccess && !rc) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess || rc || bad)
-    {
-        giveBack();
-        if (rc) return rc;
-        CK(e);
-        return fail(ctx, SKGPU_ERR_ARG, "radiation field: non-finite value");
-    }
-    if (!fits)
+    const size_t cells = ctx->numCells, nrf = ctx->nrf, len = cells * nrf;
+    if (!finiteLarge(ctx, rf, len)) return fail(ctx, SKGPU_ERR_ARG, "radiation field: non-finite value");
+    if (ctx->rfLen != len)
     {
         devFree(ctx->rf);
         devFree(ctx->rfT);
+        ctx->rfLen = 0;
+        CK(devAlloc(&ctx->rf, len));
+        ctx->rfLen = len;
     }
-    ctx->rf = tally;
-    ctx->rfT = raw;
-    ctx->rfLen = len;
-    CK(transposeField(raw, tally, ctx->nrf, ctx->numCells, ctx->stream));
+    // The caller's layout is cell-major (m * nbins + ell), the device tally wavelength-major: the device turns it,
+    // cells in parts through the kept block, so that a field takes no second field of device memory. On the
+    // host the turn and a check by one core took 19 of 21 ms for 8.6e4 cells and 50 bins.
+    const size_t rows = std::min(cells, std::max<size_t>(1, PART_DOUBLES / nrf));
+    int rc = ensurePart(ctx, rows * nrf);
+    for (size_t first = 0; first < cells && !rc; first += rows)
+    {
+        const size_t k = std::min(rows, cells - first);
+        if ((rc = copyIn(ctx, rf + first * nrf, k * nrf, ctx->part))) break;
+        CK(transposeField(ctx->part, ctx->rf + first, ctx->nrf, static_cast<int>(k), ctx->numCells, ctx->stream));
+    }
+    if (rc) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     return SKGPU_OK;
 }
@@ -2426,7 +2426,7 @@ int skgpu_fetch_radiation_field(skgpu_ctx* ctx, double* rf)
     // the device tally is wavelength-major (ell * cells + m); the caller's layout is cell-major
     int cells = static_cast<int>(ctx->rfLen / ctx->nrf), nbins = ctx->nrf;
     if (!ctx->rfT) CK(devAlloc(&ctx->rfT, ctx->rfLen));
-    CK(transposeField(ctx->rf, ctx->rfT, cells, nbins, ctx->stream));
+    CK(transposeField(ctx->rf, ctx->rfT, cells, nbins, nbins, ctx->stream));
     return addInto(ctx, ctx->rfT, ctx->rfLen, rf);
 }
 
@@ -2562,23 +2562,16 @@ int skgpu_optical_depths(skgpu_ctx* ctx, int32_t num_rays, const double* rays, d
     if (num_rays == 0) return SKGPU_OK;
     // DustMix::sectionExt(lambda) = sigma_ext[locateClip(lambda borders, lambda)]
     double section = ctx->mixExtHost[std::max(0, skg::locateClip(ctx->mixLbHost.data(), ctx->nmix, lambda))];
-    // rays and depths in device memory that the context keeps, at most 32 MB of it; a larger number of rays
-    // goes through it in parts
-    const size_t perRay = 7 * sizeof(double), rows = std::min<size_t>(num_rays, (size_t(32) << 20) / perRay);
-    if (ctx->rayRows < rows)
-    {
-        devFree(ctx->rayDev);
-        ctx->rayRows = 0;
-        CK(devAlloc(&ctx->rayDev, 7 * rows));
-        ctx->rayRows = rows;
-    }
-    double *dRays = ctx->rayDev, *dTau = dRays + 6 * rows;
+    // 7 doubles a ray (the ray and its depth), in parts through the kept block
+    const size_t rows = std::min<size_t>(num_rays, PART_DOUBLES / 7);
+    int rc = ensurePart(ctx, 7 * rows);
+    if (rc) return rc;
+    double *dRays = ctx->part, *dTau = dRays + 6 * rows;
     CK(cudaMemsetAsync(ctx->errFlag, 0, sizeof(int), ctx->stream));
     for (size_t first = 0; first < static_cast<size_t>(num_rays); first += rows)
     {
         const int k = static_cast<int>(std::min(rows, num_rays - first));
-        int rc = copyIn(ctx, rays + 6 * first, 6 * static_cast<size_t>(k), dRays);
-        if (rc) return rc;
+        if ((rc = copyIn(ctx, rays + 6 * first, 6 * static_cast<size_t>(k), dRays))) return rc;
         cudaError_t e = (precision == SKGPU_PREC_FP32 ? launchOpticalDepthsFP32 : launchOpticalDepthsFP64)(
             precision, ctx->g, ctx->dens, section, k, dRays, dTau, ctx->errFlag, ctx->stream);
         if (e != cudaSuccess) return fail(ctx, SKGPU_ERR_CUDA, std::string("optical depths: ") + cudaGetErrorString(e));

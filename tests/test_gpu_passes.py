@@ -182,7 +182,7 @@ def test_statistics_buffers_of_growing_runs(golden, gpu_backend, oracle_backend)
 @pytest.mark.parametrize("n", [1, 2, 1365, 1366, 87381, 87382, 599186, 599187, 1200001])
 def test_optical_depths_in_parts(golden, gpu_backend, n):
     """Around the direct copies (64 KB: 1 365 rays of 48 bytes), the 4 MB chunks of the pinned ones (87 381)
-    and the device block (32 MB: 599 186 rays of 56 bytes)."""
+    and the device block (32 MB: 599 186 rays and depths of 56 bytes)."""
     z = golden("paths_cartesian_c16.npz")
     sc = Scene.from_export(z)
     sc.upload(gpu_backend)
@@ -205,6 +205,30 @@ def test_radiation_field_round_trip(golden, gpu_backend, bins):
     bad.flat[-1] = np.inf
     with pytest.raises(SkgpuError):
         gpu_backend.upload_radiation_field(bad)
+    assert np.array_equal(gpu_backend.fetch_radiation_field(rf.size).reshape(rf.shape), rf)
+
+
+def test_radiation_field_takes_its_own_size_of_device_memory(golden, gpu_backend):
+    """Fields of 256 and 320 MB, in turn: the device holds the present one and a part's block (32 MB), no second
+    field and nothing of the one before. Cells and bins that do not divide a part."""
+    import torch
+    sc = Scene.from_export(golden("shell_c16.npz"))
+    sc.upload(gpu_backend)
+    cells = len(sc.density)
+
+    def upload(bins):
+        gpu_backend.upload_rf_grid(bins, np.linspace(1e-7, 1e-5, bins + 1), np.r_[-1, np.arange(bins), -1].astype(np.int32))
+        rf = np.arange(cells * bins, dtype=float).reshape(cells, bins)
+        gpu_backend.upload_radiation_field(rf)
+        return rf
+
+    upload(1)
+    torch.cuda.mem_get_info(0)  # the first query sets up torch's own CUDA state
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info(0)[0]
+    for mb in (256, 320, 256):
+        rf = upload(mb * (1 << 20) // (8 * cells) + 1)
+        assert free - torch.cuda.mem_get_info(0)[0] <= rf.nbytes + (64 << 20)
     assert np.array_equal(gpu_backend.fetch_radiation_field(rf.size).reshape(rf.shape), rf)
 
 
