@@ -5,14 +5,18 @@
 #include <condition_variable>
 #include <exception>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
+#include <unistd.h>
 
 namespace skg {
 
 // At most 16 host cores, started with the first large array and joined with the context. Starting
 // threads for every chunk of a read-back took as long as adding one (16 threads, 0.3 ms).
+// A process forked later has a copy of the pool but none of its threads: it takes no part of it (destroying
+// the condition variables would wait for those threads for ever), and works alone.
 class HostPool
 {
 public:
@@ -21,12 +25,18 @@ public:
     HostPool& operator=(const HostPool&) = delete;
     ~HostPool()
     {
+        if (!_shared) return;
+        if (_shared->process != getpid())
         {
-            std::lock_guard<std::mutex> lock(_mutex);
-            _stop = true;
+            _shared.release();
+            return;
         }
-        _wake.notify_all();
-        for (std::thread& t : _threads) t.join();
+        {
+            std::lock_guard<std::mutex> lock(_shared->mutex);
+            _shared->stop = true;
+        }
+        _shared->wake.notify_all();
+        for (std::thread& t : _shared->threads) t.join();
     }
 
     // runs f(begin, end) over shares of [0, n) on up to one thread per `grain` items; returns when done
@@ -34,16 +44,19 @@ public:
     {
         const size_t cores = std::max(1u, std::min(std::thread::hardware_concurrency(), 16u));
         size_t parts = std::max<size_t>(1, std::min(cores, (n + grain - 1) / grain));
+        if (parts > 1 && _shared && _shared->process != getpid()) parts = 1;
         if (parts > 1)
         {
-            std::lock_guard<std::mutex> lock(_mutex);
             try
             {
-                while (_threads.size() + 1 < parts) _threads.emplace_back([this, me = _threads.size()] { work(me); });
+                if (!_shared) _shared = std::make_unique<Shared>();
+                std::lock_guard<std::mutex> lock(_shared->mutex);
+                auto& threads = _shared->threads;
+                while (threads.size() + 1 < parts) threads.emplace_back([s = _shared.get(), me = threads.size()] { s->work(me); });
             }
             catch (const std::exception&)
             {
-                parts = _threads.size() + 1;  // no further thread to be had: the work goes to those there are
+                parts = _shared ? _shared->threads.size() + 1 : 1;  // no further thread to be had: the work goes to those there are
             }
         }
         if (parts == 1)
@@ -51,47 +64,54 @@ public:
             f(0, n);
             return;
         }
+        Shared& s = *_shared;
         {
-            std::lock_guard<std::mutex> lock(_mutex);
-            _job = &f;
-            _n = n;
-            _parts = parts;
-            _open = parts - 1;
-            ++_round;
+            std::lock_guard<std::mutex> lock(s.mutex);
+            s.job = &f;
+            s.n = n;
+            s.parts = parts;
+            s.open = parts - 1;
+            ++s.round;
         }
-        _wake.notify_all();
+        s.wake.notify_all();
         f(0, n / parts);
-        std::unique_lock<std::mutex> lock(_mutex);
-        _done.wait(lock, [this] { return _open == 0; });
+        std::unique_lock<std::mutex> lock(s.mutex);
+        s.done.wait(lock, [&s] { return s.open == 0; });
     }
 
 private:
-    void work(size_t me)
+    // what the caller and the workers share
+    struct Shared
     {
-        std::unique_lock<std::mutex> lock(_mutex);
-        size_t seen = 0;  // a thread started for a round takes part in it: the round ends only with its part
-        for (;;)
-        {
-            _wake.wait(lock, [&] { return _stop || _round != seen; });
-            if (_stop) return;
-            seen = _round;
-            const size_t part = me + 1;
-            if (part >= _parts) continue;
-            const auto* f = _job;
-            const size_t n = _n, parts = _parts;
-            lock.unlock();
-            (*f)(n / parts * part, part + 1 == parts ? n : n / parts * (part + 1));
-            lock.lock();
-            if (--_open == 0) _done.notify_one();
-        }
-    }
+        std::mutex mutex;
+        std::condition_variable wake, done;
+        std::vector<std::thread> threads;
+        const std::function<void(size_t, size_t)>* job = nullptr;
+        size_t n = 0, parts = 0, open = 0, round = 0;
+        bool stop = false;
+        const pid_t process = getpid();
 
-    std::mutex _mutex;
-    std::condition_variable _wake, _done;
-    std::vector<std::thread> _threads;
-    const std::function<void(size_t, size_t)>* _job = nullptr;
-    size_t _n = 0, _parts = 0, _open = 0, _round = 0;
-    bool _stop = false;
+        void work(size_t me)
+        {
+            std::unique_lock<std::mutex> lock(mutex);
+            size_t seen = 0;  // a thread started for a round takes part in it: the round ends only with its part
+            for (;;)
+            {
+                wake.wait(lock, [&] { return stop || round != seen; });
+                if (stop) return;
+                seen = round;
+                const size_t part = me + 1;
+                if (part >= parts) continue;
+                const auto* f = job;
+                const size_t total = n, shares = parts;
+                lock.unlock();
+                (*f)(total / shares * part, part + 1 == shares ? total : total / shares * (part + 1));
+                lock.lock();
+                if (--open == 0) done.notify_one();
+            }
+        }
+    };
+    std::unique_ptr<Shared> _shared;
 };
 
 }  // namespace skg
