@@ -232,6 +232,26 @@ def test_radiation_field_takes_its_own_size_of_device_memory(golden, gpu_backend
     assert np.array_equal(gpu_backend.fetch_radiation_field(rf.size).reshape(rf.shape), rf)
 
 
+def test_staging_memory_is_not_inherited(golden, gpu_backend):
+    """The pinned buffers of the large host arrays (two of 4 MB here) are marked as not copied to a forked process."""
+    def marked():
+        total = size = 0
+        with open("/proc/self/smaps") as f:
+            for line in f:
+                if line.startswith("Size:"):
+                    size = int(line.split()[1])
+                elif line.startswith("VmFlags:") and "dc" in line.split():
+                    total += size
+        return total
+
+    z = golden("paths_cartesian_c16.npz")
+    Scene.from_export(z).upload(gpu_backend)
+    gpu_backend.optical_depths(z["rays"][:4], 0.55e-6)  # too few for the staging buffers
+    before = marked()
+    gpu_backend.optical_depths(np.tile(z["rays"], (20, 1))[:5000], 0.55e-6)
+    assert marked() - before >= 8 << 10
+
+
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 65, 4736, 9472, 9473, 20001])
 def test_guide_gradient_batch_sizes(gpu_backend, n):
     """Tiles of 32 and 64 samples, whole and ragged, one and several per block (148 SMs: the larger tile
