@@ -214,7 +214,8 @@ int skgpu_upload_grid_cylinder3d(skgpu_ctx* ctx, int32_t num_radial_borders, con
                                  const double* z_borders, double eps, int32_t has_hole);
 /* TetraMeshSpatialGrid: vertices, per tetrahedron its 4 vertex indices, and per face the outward
  * normal, the neighbouring tetrahedron (-1 on the hull) and its face index
- * (TetraMeshSpatialGrid.hpp:107-133). */
+ * (TetraMeshSpatialGrid.hpp:107-133). Beside a neighbour the face index may be -1: it is then the
+ * neighbour's face that leads back, and without one the mesh is refused. */
 int skgpu_upload_grid_tetra(skgpu_ctx* ctx, int32_t num_vertices, const double* vertices, int32_t num_tetra,
                             const int32_t* tetra_vertices, const double* face_normals, const int32_t* face_ntetra,
                             const int32_t* face_nface, const double* extent, double eps);

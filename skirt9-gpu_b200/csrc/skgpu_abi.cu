@@ -1309,6 +1309,17 @@ int skgpu_upload_grid_tetra(skgpu_ctx* ctx, int32_t num_vertices, const double* 
         if (face_ntetra[q] >= num_tetra || face_ntetra[q] < -1) return fail(ctx, SKGPU_ERR_ARG, "tetra: neighbour out of range");
         if (face_nface[q] < -1 || face_nface[q] > 3) return fail(ctx, SKGPU_ERR_ARG, "tetra: face index out of range");
     }
+    // the records need a face index beside every neighbour: where the mesh leaves it open (-1), it is that of the
+    // neighbour's face that leads back
+    std::vector<int32_t> nface(face_nface, face_nface + 4 * nt);
+    for (size_t q = 0; q < 4 * nt; ++q)
+    {
+        if (face_ntetra[q] < 0 || nface[q] >= 0) continue;
+        const int32_t* back = face_ntetra + 4 * static_cast<size_t>(face_ntetra[q]);
+        for (int f = 3; f >= 0; --f)
+            if (back[f] == static_cast<int32_t>(q / 4)) nface[q] = f;
+        if (nface[q] < 0) return fail(ctx, SKGPU_ERR_ARG, "tetra: a neighbour without a face index has no face that leads back");
+    }
     // bounding boxes (Tetra constructor, TetraMeshSpatialGrid.cpp:54-81) and a uniform box grid
     std::vector<double> box(6 * nt);
     for (size_t t = 0; t < nt; ++t)
@@ -1365,7 +1376,7 @@ int skgpu_upload_grid_tetra(skgpu_ctx* ctx, int32_t num_vertices, const double* 
         for (int f = 0; f < 4; ++f)
         {
             int nb = face_ntetra[4 * t + f];
-            int nf = face_nface[4 * t + f];
+            int nf = nface[4 * t + f];
             r.to[f] = nb >= 0 ? 4 * nb + nf : -1;
             size_t owner = t;
             int of = f;
@@ -1403,7 +1414,7 @@ int skgpu_upload_grid_tetra(skgpu_ctx* ctx, int32_t num_vertices, const double* 
     if ((rc = gridUpload<int>(ctx, &g.teTet, tetra_vertices, 4 * nt))) return rc;
     if ((rc = gridUpload(ctx, &g.teNormals, face_normals, 12 * nt))) return rc;
     if ((rc = gridUpload<int>(ctx, &g.teNTet, face_ntetra, 4 * nt))) return rc;
-    if ((rc = gridUpload<int>(ctx, &g.teNFace, face_nface, 4 * nt))) return rc;
+    if ((rc = gridUpload<int>(ctx, &g.teNFace, nface.data(), nface.size()))) return rc;
     if ((rc = gridUpload(ctx, &g.teBox, box.data(), box.size()))) return rc;
     if ((rc = gridUpload<int>(ctx, &g.teBlkBegin, begin.data(), begin.size()))) return rc;
     if ((rc = gridUpload<int>(ctx, &g.teBlkTets, list.data(), list.size()))) return rc;

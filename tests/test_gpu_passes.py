@@ -252,6 +252,28 @@ def test_staging_memory_is_not_inherited(golden, gpu_backend):
     assert marked() - before >= 8 << 10
 
 
+@pytest.mark.parametrize("precision", [abi.PREC_FP64_EXACT, abi.PREC_FP32])
+def test_tetrahedra_with_open_face_indices(golden, gpu_backend, precision):
+    """A mesh that leaves the neighbours' face indices open (-1) walks as the complete one; one whose neighbour
+    does not lead back is refused."""
+    z = golden("paths_tetra.npz")
+    sc = Scene.from_export(z)
+    sc.upload(gpu_backend)
+    whole = gpu_backend.optical_depths(z["rays"], 0.55e-6, precision=precision)
+    nt, nf = (np.array(sc.grid[k], np.int32).reshape(-1, 4) for k in ("ntetra", "nface"))
+    sc.grid = dict(sc.grid, nface=np.where(nt >= 0, -1, nf).astype(np.int32))
+    sc.upload(gpu_backend)
+    assert np.array_equal(gpu_backend.optical_depths(z["rays"], 0.55e-6, precision=precision), whole)
+    t, f = np.argwhere(nt >= 0)[0]
+    back = nt[nt[t, f]]
+    back[back == t] = -1
+    nt[nt[t, f]] = back
+    sc.grid = dict(sc.grid, ntetra=nt)
+    with pytest.raises(SkgpuError) as e:
+        sc.upload(gpu_backend)
+    assert e.value.code == abi.ERR_ARG
+
+
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 65, 4736, 9472, 9473, 20001])
 def test_guide_gradient_batch_sizes(gpu_backend, n):
     """Tiles of 32 and 64 samples, whole and ragged, one and several per block (148 SMs: the larger tile
