@@ -140,6 +140,8 @@ struct GenBase
     // that would say so: 5 % faster for the tetrahedral production walker, no faster for the others, and
     // 1.6x slower for the FP64 tetrahedral one (its lanes no longer meet after a step)
     static constexpr bool kEndsOutside = false;
+    // shared memory that the walker takes in a block, beside which the scene table of a batch has to fit
+    static constexpr size_t kSharedBytes = 0;
     // the cell of a launched packet is found once, by the launch stage, instead of by each of its rays
     static constexpr bool kLocates = false;
     SKG_D static int locate(const GridDev&, double, double, double) { return -1; }

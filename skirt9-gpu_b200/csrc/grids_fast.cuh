@@ -42,9 +42,10 @@ struct BoxWalker : GenBase
 
     // the ray's reciprocal direction lives in a per-thread shared-memory slot (blocks of at most
     // 256 threads), which keeps the walkers' state within the registers of four resident blocks
+    static constexpr size_t kSharedBytes = 3 * 256 * sizeof(double);
     SKG_D static double* recip()
     {
-        __shared__ double slots[3][256];
+        __shared__ double slots[kSharedBytes / (256 * sizeof(double))][256];
         return &slots[0][threadIdx.x];
     }
 

@@ -305,6 +305,7 @@ __global__ void __launch_bounds__(256, Walker::kMinBlocks) traceKernel(const __g
     int sid = 0;
     extern __shared__ __align__(16) unsigned char traceSmem[];
     const Scene* table = reinterpret_cast<const Scene*>(traceSmem);
+    static_assert(BATCH_SHARED_BYTES + Walker::kSharedBytes <= 48 * 1024, "scene table of a full batch in shared memory");
     if constexpr (Multi)
     {
         const int4* src = reinterpret_cast<const int4*>(w.scenes);

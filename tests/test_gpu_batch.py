@@ -3,6 +3,8 @@ give every scene the tallies of its own solo run (same histories, same random st
 order of the FP64 atomic additions differs), on the reference-order FP64 walkers and on the
 production FP32 walkers, for tetrahedral and Cartesian grids; the launch shape changes nothing
 but speed; mismatched batches are refused."""
+import copy
+
 import numpy as np
 import pytest
 
@@ -68,6 +70,23 @@ def test_batched_tetra_scenes_equal_solo_runs(precision):
 @pytest.mark.parametrize("precision", [abi.PREC_FP64_EXACT, abi.PREC_FP32])
 def test_batched_cartesian_scenes_equal_solo_runs(precision):
     _check(*_shell_scenes(), precision)
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64_EXACT, abi.PREC_FP32])
+@pytest.mark.parametrize("grid", ["cartesian", "octree"])
+def test_largest_batches_equal_solo_runs(grid, precision):
+    """48 scenes, the largest batch: their table and the box walkers' own shared memory take all of a block's
+    48 KB."""
+    if grid == "cartesian":
+        base = workloads.shell_cartesian(8, 16)
+    else:
+        base = workloads.galaxy_octree(npix=16, nlambda=4, max_level=4, max_dust_fraction=1e-3, store_rf=False)
+    scenes = []
+    for i in range(48):
+        sc = copy.copy(base)
+        sc.density = base.density * (0.2 + 0.1 * i)
+        scenes.append(sc)
+    _check(scenes, [200 + 37 * i for i in range(48)], list(range(48)), precision)
 
 
 def test_batch_refuses_mixed_grid_kinds():
