@@ -20,7 +20,7 @@ struct GraphCache
     // the second stream of the pipelined passes and its events, created with the first captured graph
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
-    int kernelsPerPass = 0;  // of the last run
+    int kernelsPerPass = 0, kernelsOnce = 0;  // of the last run
     void reset()
     {
         if (exec) cudaGraphExecDestroy(exec);

@@ -1892,7 +1892,7 @@ static int runAndCollect(skgpu_ctx* ctx, const Wave& w, bool useGraph, bool time
     ctx->lastCounters.rf_stores = ctl.counters[4];
     ctx->lastCounters.stats_overflows = ctl.counters[5];
     ctx->lastCounters.stats_spilled = ctl.counters[6];
-    ctx->lastCounters.kernel_launches = static_cast<uint64_t>(passes) * ctx->graphCache.kernelsPerPass + 1 + (w.order ? 3 : 0);
+    ctx->lastCounters.kernel_launches = static_cast<uint64_t>(passes) * ctx->graphCache.kernelsPerPass + ctx->graphCache.kernelsOnce + (w.order ? 3 : 0);
     ctx->lastPasses = passes;
     ctx->lastGuideWeightSum = ctl.guideWeightSum;
     ctx->lastGuideEvents = ctl.guideEvents;

@@ -220,7 +220,11 @@ cudaError_t runWave(const Wave& wave, int numSMs, cudaStream_t s, unsigned long 
         cudaError_t ea = cudaFuncSetAttribute(guideScatterKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GM_SMEM_BYTES);
         if (ea != cudaSuccess) return ea;
     }
-    if (cache) cache->kernelsPerPass = (L.pipelined ? (L.forced ? 6 : 4) + (L.guided ? 1 : 0) + (w.anyStats ? 1 : 0) : 7) + (L.guided ? 1 : 0);
+    if (cache)
+    {
+        cache->kernelsPerPass = (L.pipelined ? (L.forced ? 6 : 4) + (L.guided ? 1 : 0) + (w.anyStats ? 1 : 0) : 7) + (L.guided ? 1 : 0);
+        cache->kernelsOnce = 1;
+    }
     initPoolKernel<<<L.shadeBlocks, L.threads, 0, s>>>(w, w.anyStats && clearStats ? 1 : 0);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -297,6 +301,7 @@ cudaError_t runWave(const Wave& wave, int numSMs, cudaStream_t s, unsigned long 
     if (e == cudaSuccess && L.pipelined && w.anyStats)
     {
         flushEndedKernel<<<L.shadeBlocks, L.threads, 0, s>>>(w, 1);  // the histories that the last pass ended
+        cache->kernelsOnce++;
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     }

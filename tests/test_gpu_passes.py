@@ -141,6 +141,19 @@ def test_pipelined_equals_plain_passes_of_spilled_statistics(golden, gpu_backend
     assert a.counters["stats_spilled"] > 0 and a.counters["stats_overflows"] == 0
 
 
+def test_kernel_launches_are_counted(golden, gpu_backend):
+    """The pool's initialisation and six kernels a pass; statistics take one more in each, and one after the last."""
+    launches = []
+    for stats in (0, 1):
+        sc = Scene.from_export(golden("shell_c16.npz"))
+        for ins in sc.instruments:
+            ins["stats"] = stats
+        sc.upload(gpu_backend)
+        launches.append(sc.run(gpu_backend, 5000, seed=5).counters["kernel_launches"])
+    passes, rest = divmod(launches[0] - 1, 6)
+    assert rest == 0 and launches[1] == 7 * passes + 2
+
+
 @pytest.mark.parametrize("stats", [0, 1])
 @pytest.mark.parametrize("slots", [256, 1000])
 def test_pipelined_passes_refill_a_small_pool(golden, gpu_backend, slots, stats):
