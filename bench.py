@@ -8,9 +8,10 @@ storage, scattering peel-off and HG scattering for every history. `value` is dev
 events on the launch stream, L2 flushed between steps); `e2e` is measured through the same C ABI
 with host buffers (medium state uploaded from pinned memory, every instrument tally and the
 radiation field added into the caller's host arrays, every step). The roofline is that of the
-traversal kernel, whose launches are bracketed by CUDA events inside the timed steps. Under
-torchrun each rank traces its own contiguous range of history indices (weak scaling; no
-data-path collective).
+traversal kernel of one more step after the timed ones, whose launches are bracketed by CUDA events:
+it runs the plain passes, one traversal kernel for all rays, where the timed steps run the pipelined
+ones, whose kernels overlap. Under torchrun each rank traces its own contiguous range of history
+indices (weak scaling; no data-path collective).
 """
 import argparse
 import json
@@ -380,7 +381,7 @@ def run_batch_arm(args, rank, world, local):
             ms.append(step())
             counters = be0.counters()
     torch.cuda.synchronize()
-    trace_ms, trace_launches = traversal_times(be0, step, args.steps)
+    trace_ms, trace_launches, plain = traversal_times(be0, step, args.steps)
     total_ms = max_over_ranks(float(sum(ms)), world, local)
     value = per_gpu * world * args.steps / (total_ms / 1e3)
 
@@ -410,7 +411,7 @@ def run_batch_arm(args, rank, world, local):
 
     if rank == 0:
         line = result_line(args, "batch", world, value, total_ms, trace_ms, trace_launches, counters, abi.GRID_TETRA,
-                           prec, clk, e2e, per_gpu)
+                           prec, clk, e2e, per_gpu, plain)
         line["config"]["simulations"] = n
         if n != 16 or args.packet_scale != 1.0:
             line["config"]["subset"] = f"first {n} simulations, {args.packet_scale:g} of their packets (profiling case)"
@@ -440,31 +441,35 @@ def max_over_ranks(x, world, local):
 def traversal_times(be, step, steps):
     """Device milliseconds and launches of the traversal kernel in `steps` steps, from one more step with
     CUDA events around every launch (after the timed ones: it runs the plain passes, whose single
-    traversal kernel can be timed, where the timed steps run the pipelined ones)."""
+    traversal kernel can be timed, where the timed steps run the pipelined ones), and that step's own
+    milliseconds and counters."""
     from skgpu import abi
     abi.set_stage_timing(be, 1)
     try:
-        step()
+        step_ms = step()
         ms, launches = abi.last_stage_times(be)["trace"]
+        counters = be.counters()
     finally:
         abi.set_stage_timing(be, 0)
-    return ms * steps, launches * steps
+    return ms * steps, launches * steps, {"ms": step_ms, "counters": counters}
 
 
 def result_line(args, name, world, value, total_ms, trace_ms, trace_launches, counters, kind, prec, clk, e2e,
-                per_gpu):
-    """The JSON line of our arm; the roofline is that of the traversal kernel: its algorithmic bytes per
-    launch over its average launch duration (CUDA events on the launch stream, in one extra step of plain passes)."""
+                per_gpu, plain=None):
+    """The JSON line of our arm; the roofline is that of the traversal kernel of the plain passes (mode 0): its
+    algorithmic bytes per launch over its average launch duration (CUDA events on the launch stream, in one
+    extra step: `plain`, with that step's milliseconds and counters)."""
     from skgpu import abi
     peak, peak_kind = peaks()
-    trace_bytes_per_launch = trace_algorithmic_bytes(counters, kind) / max(1, trace_launches / args.steps)
+    plain = plain or {"ms": None, "counters": counters}
+    trace_bytes_per_launch = trace_algorithmic_bytes(plain["counters"], kind) / max(1, trace_launches / args.steps)
     trace_avg_ms = trace_ms / max(1, trace_launches)
     achieved = trace_bytes_per_launch / (trace_avg_ms / 1e3) / 1e9
     traffic, profile = None, {}
     prof = os.path.join(ROOT, "profiles", f"trace_kernel_{name}_{args.precision}.json")
     if os.path.exists(prof):
         with open(prof) as f:
-            profile = json.load(f)
+            profile = json.load(f).get("plain_passes", {})
         ratio = profile.get("dram_bytes_per_algorithmic_byte")
         if ratio:
             traffic = ratio * trace_bytes_per_launch
@@ -478,11 +483,11 @@ def result_line(args, name, world, value, total_ms, trace_ms, trace_launches, co
                    "parallelism": f"history ranges x{world}" if name != "batch" else f"independent batches x{world}"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "peak_kind": peak_kind,
-                     "kernel": profile.get("kernel", "skg::traceKernel"),
+                     "kernel": profile.get("kernel", "skg::traceKernel, mode 0"),
+                     "scope": "plain passes of one extra step; the timed steps run the pipelined passes",
                      "launches_per_step": trace_launches / args.steps, "avg_launch_ms": trace_avg_ms,
                      "algorithmic_bytes_per_launch": trace_bytes_per_launch,
-                     # of the plain passes' traversal, over the timed (pipelined) step
-                     "share_of_step": trace_ms / max(total_ms, 1e-9),
+                     "share_of_step": trace_ms / args.steps / plain["ms"] if plain["ms"] else None,
                      # what ncu shows limits it (profiles/): the algorithmic bytes come mostly from L2
                      "limiter": profile.get("limiter"), "l2_throughput_frac": profile.get("l2_throughput_frac"),
                      "dram_throughput_frac": profile.get("dram_throughput_frac")},
@@ -737,7 +742,7 @@ def main():
             ms.append(step())
             counters = be.counters()
     torch.cuda.synchronize()
-    trace_ms, trace_launches = traversal_times(be, step, args.steps)
+    trace_ms, trace_launches, plain = traversal_times(be, step, args.steps)
     total_ms = max_over_ranks(float(sum(ms)), world, local)
     value = npp_total * args.steps / (total_ms / 1e3)
 
@@ -784,7 +789,7 @@ def main():
 
     if rank == 0:
         line = result_line(args, name, world, value, total_ms, trace_ms, trace_launches, counters, sc.grid["kind"],
-                           prec, clk, e2e, per_gpu)
+                           prec, clk, e2e, per_gpu, plain)
         if not args.no_cpu_baseline:
             try:
                 line["cpu_baseline"] = cpu_baseline(name)

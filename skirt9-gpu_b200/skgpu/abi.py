@@ -533,7 +533,8 @@ STAGES = ("trace", "peel", "prop1", "prop2", "free", "guide", "launch")  # SKGPU
 
 
 def set_stage_timing(be, level):
-    """CUDA-event timing of the stage kernels of later runs: 0 off, 1 traversal kernel, 2 all stages."""
+    """CUDA-event timing of the stage kernels of later runs: 0 off, 1 traversal kernel, 2 all stages. Timed runs
+    take the plain passes, whose stages do not overlap."""
     f = be.lib.skgpu_set_stage_timing
     f.argtypes = [C.c_void_p, C.c_int32]
     f.restype = C.c_int

@@ -50,5 +50,26 @@ def test_result_line_carries_the_contract_keys():
     assert line["config"]["workload"] == "galaxy" and line["higher_is_better"] is True
 
 
+def test_roofline_describes_the_step_that_was_timed_for_it():
+    """Kernel, bytes, traffic and share are those of the extra step of plain passes, not of the timed steps."""
+    args = argparse.Namespace(steps=5, warmup=3, precision="fp32", gpus=1)
+
+    class Clk:
+        def summary(self):
+            return {"sm_mhz": 1965.0, "sm_max_mhz": 1965.0, "reasons": []}
+
+    timed, extra = _counters(crossings=999), _counters()
+    for name, kind in (("galaxy", 1), ("voronoi", 2), ("batch", 3), ("shell", 0)):
+        line = bench.result_line(args, name, 1, 2.0e7, 5000.0, 4000.0, 100, timed, kind, 1, Clk(), None, 10 ** 8,
+                                 {"ms": 900.0, "counters": extra})
+        rf = line["roofline"]
+        assert rf["share_of_step"] == 800.0 / 900.0
+        per_launch = bench.trace_algorithmic_bytes(extra, kind) / 20
+        assert rf["algorithmic_bytes_per_launch"] == per_launch
+        assert "plain passes" in rf["scope"] and "mode 0" in rf["kernel"]
+        assert rf["traffic"] is None or 0 < rf["traffic"] < 2 * per_launch
+        assert line["counters_per_step"] == timed
+
+
 def test_max_over_ranks_is_identity_on_one_rank():
     assert bench.max_over_ranks(3.5, 1, 0) == 3.5
