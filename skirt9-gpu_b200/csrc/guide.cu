@@ -48,10 +48,12 @@ SKG_D void mlpForward(const float* P, const float* in, float* h /*4 x 64*/, floa
 // so that the reads of a warp fall on different banks. The blocks' sums go to `partial` and
 // gradSumKernel adds them, in block order: the result does not depend on timing.
 //
-// 12 wavefronts of shared memory per 64 multiply-adds of a warp, so the multiply-adds bound it: 1.5
+// 12 wavefronts of shared memory per 64 multiply-adds of a warp, so the multiply-adds bound a tile: 1.5
 // GFLOP for 16 384 samples. One thread per sample with its activations in local memory, and one thread
-// per parameter that went over the whole batch, took 1.9 ms for them, copies and all 2.05 ms; now the
-// call takes 0.21 ms (B200), most of it the copies of its host arrays.
+// per parameter that went over the whole batch, took 1.9 ms for them, copies and all 2.05 ms. Now the kernel
+// and the sum of its blocks take 94 us, measured as a step of training (B200): 29 us for each of a block's
+// two tiles, at 40 % of the multiply-add rate, and some 35 us for the launches, the network's way into
+// shared memory and the blocks' sums out of it. guideLossGrad takes 0.21 ms with the copies of its host arrays.
 // ---------------------------------------------------------------------------------------------
 constexpr int GB_THREADS = 256;
 constexpr int GB_LD = 68, GB_LD0 = 12;  // row lengths in floats: 64-wide rows, and the 8 inputs
@@ -444,10 +446,12 @@ cudaError_t allocN(T** p, size_t n)
 }
 
 // Tiles of 64 samples, which read shared memory half as often per multiply-add, or of 32 for a batch of
-// at most 64 per SM: a block then has one tile of either size, and the small one is done sooner.
+// at most 32 per SM: a block then has one tile of either size, and the small one is done sooner. A step of
+// training with tiles of 32 / 64: 500 samples 43 / 53 us, 4736 (32 per SM) 53 / 59, 4737 72 / 59, 9472 73 / 65, 16 384
+// 111 / 94.
 cudaError_t launchBatch(GuideState* g, int n, const BatchSource& src, int numSMs, int* blocks)
 {
-    const bool small = n <= 64 * numSMs;
+    const bool small = n <= 32 * numSMs;
     const int S = small ? 32 : 64;
     const size_t bytes = gbFloats(S) * sizeof(float);
     const void* f = small ? reinterpret_cast<const void*>(batchKernel<32>) : reinterpret_cast<const void*>(batchKernel<64>);

@@ -296,10 +296,10 @@ def test_tetrahedra_with_open_face_indices(golden, gpu_backend, precision):
     assert e.value.code == abi.ERR_ARG
 
 
-@pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 65, 4736, 9472, 9473, 20001])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 65, 4736, 4737, 9472, 9473, 20001])
 def test_guide_gradient_batch_sizes(gpu_backend, n):
     """Tiles of 32 and 64 samples, whole and ragged, one and several per block (148 SMs: the larger tile
-    from 9 473 samples on). FP32 sums of n terms of about one size: 1e-5 of the largest entry."""
+    from 4 737 samples on, two of them from 9 473 on). FP32 sums of n terms of about one size: 1e-5 of the largest entry."""
     import guide_oracle as go
     from test_gpu_guide import _batch
     p = go.random_params(4).astype(np.float32)
