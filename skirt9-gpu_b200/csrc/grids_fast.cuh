@@ -41,7 +41,8 @@ struct BoxWalker : GenBase
     double xE, yE, zE;  // exit walls of the current cell
 
     // the ray's reciprocal direction lives in a per-thread shared-memory slot (blocks of at most
-    // 256 threads), which keeps the walkers' state within the registers of four resident blocks
+    // 256 threads): six registers less per thread. Of the FP32 kernels at four blocks per SM (64 registers)
+    // the Cartesian ones then spill nothing, the octree's 20 (peel-off rays) to 64 bytes (forced paths).
     static constexpr size_t kSharedBytes = 3 * 256 * sizeof(double);
     SKG_D static double* recip()
     {

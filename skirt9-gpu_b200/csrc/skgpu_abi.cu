@@ -158,7 +158,8 @@ int syncLeafDensity(skgpu_ctx* ctx)
 // histories in flight at most; a larger range streams through the pool
 constexpr uint64_t POOL_DEFAULT = 1u << 22;  // packet slots in flight unless a launch shape sets them
 constexpr uint64_t POOL_MAX = 1u << 22;
-// wavefront passes per run at most (each history needs about two passes per scattering event)
+// wavefront passes per run at most (a history takes one pass per scattering event, two in plain passes of forced
+// propagation)
 constexpr long long MAX_PASSES = 2LL * MAX_SCATT_EVENTS + 64;
 
 template<typename T>
@@ -2356,7 +2357,6 @@ int skgpu_run_primary_noalloc(skgpu_ctx* ctx, uint64_t first, uint64_t count, ui
     return runAndCollect(ctx, w, false, false);
 }
 
-// host[i] += src[i] for i < n, split over the host cores for large n
 int skgpu_fetch_instrument(skgpu_ctx* ctx, int32_t instrument, double* ifu, double* sed, double* ifu_stats,
                            double* sed_stats)
 {

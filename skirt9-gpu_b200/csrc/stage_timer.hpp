@@ -7,10 +7,11 @@ namespace skg {
 
 // Optional device timing of the stage kernels with CUDA events on the launch stream. Level 1 times
 // the trace kernel only (two events per pass), level 2 every stage (eight events per pass: before
-// the trace kernel and after each stage; launch preparation and launch count as one stage). In a
-// captured graph the events become event-record nodes; they are read after every batch, once the
-// stream has synchronised, and summed into ms / launches in the order of SKGPU_STAGE_*. Stages
-// that a run does not launch (the guided-scattering stage without guiding) are not counted.
+// the trace kernel and after each stage; launch preparation and launch count as one stage). A timed
+// run takes the plain passes; in their captured graph the events become event-record nodes. They are
+// read after every batch, once the stream has synchronised, and summed into ms / launches in the order
+// of SKGPU_STAGE_*. Stages that a run does not launch (the guided-scattering stage without guiding) are
+// not counted.
 struct StageTimer
 {
     static constexpr int kBatch = 4;

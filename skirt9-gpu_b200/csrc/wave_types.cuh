@@ -63,7 +63,7 @@ struct PacketPool
 struct TaskBuf
 {
     int* slot;
-    int* info;      // PEEL: first instrument of the observer group | numScatt << 8
+    int* info;      // PEEL: first instrument of the observer group | scene << 8 | numScatt << 14
     double* par;    // PEEL: peel-off luminosity; PROP2/FREE: interaction optical depth
     double *x, *y, *z;  // PEEL: origin (the packet position at the event)
     // PEEL, pipelined passes: what the ray needs of its packet, whose slot may by then hold another one

@@ -11,7 +11,8 @@
 //          (MonteCarloSimulation::simulateForcedPropagation :1492-1546, SpatialGridPath::findInteractionPoint :161-203)
 //   FREE   non-forced propagation (simulateNonForcedPropagation :1996-2030,
 //          MediumSystem::setInteractionPointUsingExtinction :2005-2150)
-// One pass of the wavefront runs:
+// One plain pass of the wavefront runs (the pipelined passes of untimed runs take the same steps in other
+// launches, see wavefront_driver.cuh):
 //   trace    a persistent kernel: each lane takes a task, walks its ray to the end (one cell
 //            crossing per loop iteration, so the warp's lanes stay converged on the crossing code);
 //            a warp takes new task indices with one atomic once enough of its lanes wait;

@@ -57,7 +57,7 @@ void launchTrace(const Wave& w, int cur, int blocks, const WaveLaunch& L, cudaSt
 // rays of one traversal run beside the next one instead of alone. Only where the pilot records of a
 // history are closed at its end do its detections come first (`strict`).
 // The plain pass below walks the forced paths and the searches in passes of their own (twice the
-// passes, each as long as its longest ray), joins its streams in each, and takes eight kernels.
+// passes, each as long as its longest ray), on one stream, in seven kernels.
 template<class Walker>
 cudaError_t enqueuePipelined(const Wave& w, int pass, const WaveLaunch& L, cudaStream_t s)
 {
@@ -117,13 +117,6 @@ cudaError_t enqueuePass(const Wave& w, int pass, const WaveLaunch& L, cudaStream
     return cudaGetLastError();
 }
 
-// Runs histories [w.first, w.first + w.count). `doneHost` receives the progress word (pinned host
-// memory for the graph path). With `useGraph` the passes are captured once into a CUDA graph of
-// four passes and replayed; without it the same kernels are launched directly (no graph objects are
-// created). Returns a CUDA error, or cudaErrorLaunchTimeout (mapped to SKGPU_ERR_TIMEOUT) when the
-// pass limit is reached without finishing. `passes` receives the number of passes run.
-// the inputs a captured pass graph depends on: the wave parameters (by value in every kernel
-// node), the launch shape, the walker and the timing events recorded into it
 // the pipelined passes are on unless SKGPU_SPLIT_TRAVERSAL=0 (a switch for comparing the two forms)
 inline bool pipelinedPasses()
 {
@@ -164,6 +157,8 @@ void applyTraceCarveout()
     set(reinterpret_cast<const void*>(&traceKernel<Walker, true, TRACE_SEARCH>));
 }
 
+// the inputs a captured pass graph depends on: the wave parameters (by value in every kernel
+// node), the launch shape, the walker and the timing events recorded into it
 template<class Walker>
 std::vector<unsigned char> graphKey(const Wave& w, const WaveLaunch& L, const StageTimer* timer)
 {
@@ -182,6 +177,11 @@ std::vector<unsigned char> graphKey(const Wave& w, const WaveLaunch& L, const St
     return k;
 }
 
+// Runs histories [w.first, w.first + w.count). `doneHost` receives the progress word (pinned host
+// memory for the graph path). With `useGraph` the passes are captured once into a CUDA graph of
+// four passes and replayed; without it the same kernels are launched directly (no graph objects are
+// created). Returns a CUDA error, or cudaErrorLaunchTimeout (mapped to SKGPU_ERR_TIMEOUT) when the
+// pass limit is reached without finishing. `passes` receives the number of passes run.
 template<class Walker>
 cudaError_t runWave(const Wave& wave, int numSMs, cudaStream_t s, unsigned long long* doneHost, long long* passes,
                     long long maxPasses, bool useGraph, StageTimer* timer, GraphCache* cache, bool clearStats)
@@ -290,8 +290,9 @@ cudaError_t runWave(const Wave& wave, int numSMs, cudaStream_t s, unsigned long 
             lastDone = *doneHost;
             lastProgress = *passes;
         }
-        // no history finished for 65536 passes (more than 32768 scattering events of one history),
-        // or the overall pass limit: stop with a timeout status instead of looping on
+        // no history finished for 65536 passes (as many scattering events of one history with pipelined passes
+        // or free propagation, half as many in plain passes of forced ones), or the overall pass limit: stop
+        // with a timeout status instead of looping on
         if (*passes >= maxPasses || *passes - lastProgress > 65536)
         {
             e = cudaErrorLaunchTimeout;

@@ -1,10 +1,10 @@
 """GPU tests of the measurement aids and the tally read-back of the C ABI.
 
 - Stage timing (skgpu_set_stage_timing / skgpu_last_stage_times) brackets the stage kernels with
-  CUDA events inside the captured graph; it must not change the results, every stage must report
-  one launch per pass, and the stage times must add up to at most the run's device time.
-- Tallies larger than one pinned staging chunk (8M doubles) are read back in pipelined chunks and
-  added into the caller's arrays; a 512x512x40 frame spans two chunks, and the result must still
+  CUDA events inside the captured graph of plain passes; it must not change the results, every stage must
+  report one launch per pass, and the stage times must add up to at most the run's device time.
+- Tallies larger than one pinned staging chunk (0.5 to 4M doubles) are read back in pipelined chunks and
+  added into the caller's arrays; a 512x512x40 frame spans several, and the result must still
   equal the oracle's history by history, and a second fetch into the same array must double it.
 """
 import numpy as np
@@ -47,7 +47,7 @@ def test_stage_timing_level_one_times_trace_only(golden, gpu_backend):
     finally:
         abi.set_stage_timing(gpu_backend, 0)
     assert list(stages) == ["trace"]
-    # one traversal stage per pass; a pass is 8 kernels with the split traversal of the captured graph
+    # one traversal stage per pass; a plain pass is 7 kernels, 8 with guiding
     passes = stages["trace"][1]
     assert res.counters["kernel_launches"] - 1 in (7 * passes, 8 * passes)
     with pytest.raises(abi.SkgpuError):
