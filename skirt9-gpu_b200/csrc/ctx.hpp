@@ -83,6 +83,7 @@ struct skgpu_ctx
     // pinned staging of the large host arrays: the copy of one chunk overlaps the host's work on another
     double* pin[2] = {nullptr, nullptr};
     size_t pinDoubles = 0;
+    size_t unstaged = 0;  // doubles copied without them
     cudaEvent_t pinEv[2] = {nullptr, nullptr};
     skg::HostPool pool;
     // device block of the calls that work in parts (rays and depths, a field on its way to the tally)

@@ -204,14 +204,16 @@ def test_statistics_buffers_of_growing_runs(golden, gpu_backend, oracle_backend)
 @pytest.mark.parametrize("n", [1, 2, 1365, 1366, 87381, 87382, 599186, 599187, 1200001])
 def test_optical_depths_in_parts(golden, gpu_backend, n):
     """Around the direct copies (64 KB: 1 365 rays of 48 bytes), the 4 MB chunks of the pinned ones (87 381)
-    and the device block (32 MB: 599 186 rays and depths of 56 bytes)."""
+    and the device block (32 MB: 599 186 rays and depths of 56 bytes): as a context's first calls, which copy
+    directly, and after a call that moves more than 64 MB, through the pinned buffers."""
     z = golden("paths_cartesian_c16.npz")
     sc = Scene.from_export(z)
     sc.upload(gpu_backend)
     rays = z["rays"]
     few = gpu_backend.optical_depths(rays, 0.55e-6)
-    at = np.arange(n) % len(rays)
-    assert np.array_equal(gpu_backend.optical_depths(rays[at], 0.55e-6), few[at])
+    for k in (n, 1300000, n):
+        at = np.arange(k) % len(rays)
+        assert np.array_equal(gpu_backend.optical_depths(rays[at], 0.55e-6), few[at])
 
 
 @pytest.mark.parametrize("bins", [1, 31, 32, 33, 70])
@@ -268,10 +270,26 @@ def test_staging_memory_is_not_inherited(golden, gpu_backend):
 
     z = golden("paths_cartesian_c16.npz")
     Scene.from_export(z).upload(gpu_backend)
-    gpu_backend.optical_depths(z["rays"][:4], 0.55e-6)  # too few for the staging buffers
+    rays = np.tile(z["rays"], (4200, 1))
+    gpu_backend.optical_depths(rays[:100000], 0.55e-6)  # 6 MB: copied directly
     before = marked()
-    gpu_backend.optical_depths(np.tile(z["rays"], (20, 1))[:5000], 0.55e-6)
+    gpu_backend.optical_depths(rays, 0.55e-6)  # 70 MB more
     assert marked() - before >= 8 << 10
+
+
+def test_a_first_call_pins_nothing_for_a_few_rays(golden, gpu_backend):
+    """What a context pays for its staging buffers: nothing before it has copied 64 MB or fetched a large tally."""
+    def pinned():
+        with open("/proc/self/smaps") as f:
+            return sum("dc" in line.split() for line in f if line.startswith("VmFlags:"))
+
+    z = golden("paths_cartesian_c16.npz")
+    Scene.from_export(z).upload(gpu_backend)
+    gpu_backend.optical_depths(z["rays"][:4], 0.55e-6)
+    before = pinned()
+    for n in (1400, 30000, 300000):
+        gpu_backend.optical_depths(z["rays"][np.arange(n) % len(z["rays"])], 0.55e-6)
+    assert pinned() == before
 
 
 @pytest.mark.parametrize("precision", [abi.PREC_FP64_EXACT, abi.PREC_FP32])
